@@ -117,18 +117,26 @@ def _normal(rows, cols, dtype, g, pad=True):
 
 
 def _potential(side, wells, g):
-    """Sum of Gaussian wells (depth 1 to 5, width 2 to 6 grid units), or uniform in [0, 1)
-    when ``wells`` is 0; x fastest."""
+    """Sum of Gaussian wells (depth 1 to 5, width 2 to 6 grid units), one to a cell of the
+    box, as atoms keep apart: one structure, of which every seed is another configuration
+    (wells displaced by up to a grid unit, depths by 2 %). Uniform in [0, 1) when ``wells``
+    is 0. x fastest."""
     n = side ** 3
     if wells == 0:
         return torch.rand(n, generator=g, device="cuda", dtype=torch.float64)
-    u = torch.rand(wells, 5, generator=g, device="cuda", dtype=torch.float64).cpu()
+    u = torch.rand(wells, 5, generator=torch.Generator().manual_seed(5), dtype=torch.float64)
+    moved = torch.rand(wells, 4, generator=g, device="cuda", dtype=torch.float64).cpu() * 2 - 1
     x = torch.arange(side, device="cuda", dtype=torch.float64)
     v = torch.zeros(side, side, side, device="cuda", dtype=torch.float64)
+    cells = math.ceil(round(wells ** (1.0 / 3.0), 9))
     for k in range(wells):
-        a, w = 1.0 + 4.0 * float(u[k, 0]), 2.0 + 4.0 * float(u[k, 1])
-        e = [torch.exp(-(x - float(u[k, 2 + i]) * (side - 1)) ** 2 / (2.0 * w * w))
-             for i in range(3)]
+        a = (1.0 + 4.0 * float(u[k, 0])) * (1.0 + 0.02 * float(moved[k, 0]))
+        w = 2.0 + 4.0 * float(u[k, 1])
+        e = []
+        for i in range(3):
+            cell = k // cells ** i % cells
+            at = (cell + float(u[k, 2 + i])) / cells * (side - 1) + float(moved[k, 1 + i])
+            e.append(torch.exp(-(x - at) ** 2 / (2.0 * w * w)))
         v -= a * e[2][:, None, None] * e[1][None, :, None] * e[0][None, None, :]
     return v.reshape(-1)
 
@@ -230,13 +238,11 @@ def prepare(case, seed):
         o = fe.fasteig_options(A.rows)
         for k, v in dict(solver=case["solver"], nev=case["nev"], block=case["block"],
                          degree=case["degree"], which="SR", tol=1e-8, maxiter=300,
-                         precision=case["precision"], seed=1).items():
+                         precision=case["precision"], seed=1 + int(seed) % 1000000).items():
             o.set(k, v)
         if case["solver"] == "Chebyshev":
-            for k, v in dict(bounds="ritz", amplification=1e6, locking="hard",
-                             mixed_switch=1e-6).items():
+            for k, v in dict(bounds="ritz", amplification=1e6, init="device").items():
                 o.set(k, v)
-            o.set("init", "device")
         return dict(problem=fe.fasteig_problem(A, solver=case["solver"]), options=o)
     s = _blocks(case, seed)
     if kind in ("spmm", "filter"):
