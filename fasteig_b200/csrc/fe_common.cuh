@@ -102,6 +102,9 @@ struct Csr {
   // max |column - row| over the stored entries, measured on first use by the
   // multi-step filter (-1: not measured yet)
   mutable int64_t bandwidth = -1;
+  // Rows from line to line and from plane to plane of the grid that the diagonals show
+  // (csr_find_grid; 0: none seen). Orders the row blocks of spmm_rows.cu, nothing else.
+  int grid_s1 = 0, grid_s2 = 0;
   // SpMM kernel chosen by fe_csr_autotune per precision (0 FP64, 1 FP32) for up
   // to four block widths; mode < 0 marks an empty entry.
   struct Tuned {
@@ -112,6 +115,18 @@ struct Csr {
 };
 
 int num_sms();
+
+// The grid behind the operator's diagonals, from a few rows of it on the host (rowptr and
+// colind start at row `row0`) or on the device (spmm_rows.cu).
+void csr_find_grid(Csr& A, const int32_t* rowptr, const int32_t* colind, int64_t row0,
+                   int64_t count);
+void csr_find_grid_device(Csr& A);
+// Y = alpha A X + gamma X + beta Z (+ R diag(delta) if R), several rows to a warp
+// (spmm_rows.cu); false, with nothing launched, where it does not apply.
+template <typename T>
+bool csr_spmm_rows(const Csr& A, const T* X, int64_t ldx, T* Y, int64_t ldy, const T* Z,
+                   int64_t ldz, const T* R, int64_t ldr, const T* delta, int64_t ncols,
+                   double alpha, double gamma, double beta, cudaStream_t s);
 
 // Device status word that kernels launched from this host thread record a
 // timed-out bounded wait in: the one a solve installed for its duration

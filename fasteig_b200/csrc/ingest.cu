@@ -387,6 +387,7 @@ Csr* csr_from_triplets(int64_t n, int64_t count, const int32_t* rows, const int3
     FE_CHECK_CUDA(cudaMemcpyAsync(&mx_h, mx.p, sizeof(int), cudaMemcpyDeviceToHost, s));
     FE_CHECK_CUDA(cudaStreamSynchronize(s));
     A->max_row_nnz = mx_h;
+    csr_find_grid_device(*A);
   } catch (...) {
     cudaFree(A->rowptr);
     cudaFree(A->colind);

@@ -1199,6 +1199,9 @@ void csr_spmm_mode(int mode, const Csr& A, const T* X, int64_t ldx, T* Y, int64_
   }
   FE_REQUIRE(!ranges_overlap(X, A.cols, ldx, ncols, static_cast<const T*>(Y), A.rows, ldy, ncols),
              "csr_spmm: X and Y overlap");
+  if (mode == 0 && csr_spmm_rows<T>(A, X, ldx, Y, ldy, Z, ldz, nullptr, 0, nullptr, ncols, alpha,
+                                    gamma, beta, s))
+    return;
   const T* vals = nullptr;
   if constexpr (sizeof(T) == 8) vals = A.val64; else vals = A.val32;
   constexpr int VEC = VecT<T>::width;
@@ -1346,6 +1349,10 @@ void csr_spmm_corr_f32(const Csr& A, const float* X, int64_t ldx, float* Y, int6
                        cudaStream_t s) {
   if (ncols == 0 || A.rows == 0) return;
   FE_REQUIRE(R && delta && ldr >= ncols, "csr_spmm_corr: invalid correction block");
+  if (X && Y && ldx >= ncols && ldy >= ncols && (beta == 0.0 || (Z && ldz >= ncols)) &&
+      !ranges_overlap(X, A.cols, ldx, ncols, static_cast<const float*>(Y), A.rows, ldy, ncols) &&
+      csr_spmm_rows<float>(A, X, ldx, Y, ldy, Z, ldz, R, ldr, delta, ncols, alpha, gamma, beta, s))
+    return;
   constexpr int VEC = 2;  // 8-byte lanes, as the default row kernel
   constexpr int NZ = 7;
   const bool ub = beta != 0.0;

@@ -1,0 +1,543 @@
+// Block SpMM and Chebyshev step with several rows to a warp, over bricks of the grid that
+// the operator's diagonals show (sm_100a).
+//
+// A group of G lanes owns a row and reads 16 bytes a lane, so a warp works on 32 / G rows
+// of one column panel (256 or 128 bytes of every row). What bounds it, after DRAM, is the
+// instructions and the load-store wavefronts of an SM rather than the bytes: one warp per
+// row with 8-byte lanes spends them on a row of few columns as on a wide one (96^3 grid,
+// 7 points, FP32 step of 64 columns: 380 us so, 161 us here, 113 us of DRAM traffic at the
+// copy rate). Hence 16-byte lanes, byte pitches in 32 bits (one wide multiply-add per
+// address), all neighbours of a row in flight, and no predicates where the rows of the
+// warp have as many entries.
+//
+// Rows are dealt out in bricks: a CTA's groups take bx x by rows of neighbouring lines and
+// sweep down bz planes, so that the neighbours along a line, across lines and from plane to
+// plane are read while L1 still holds them: 57 % of the loads hit L1 against 24 % for
+// consecutive rows (128^3, FP32 step of 320 columns: 1.91 ms with one warp per row, 2.35 ms
+// with consecutive rows here, 1.70 ms in bricks, 1.27 ms of DRAM traffic). The brick is
+// only an order: any strides s1 (line) and s2 (plane, a multiple of s1) number every row
+// once.
+//
+// A row's arithmetic is that of the kernel of spmm.cu which such a block would have there,
+// bit for bit: with FOLD, alpha and gamma are folded into the coefficients (the row
+// kernel); without, they are applied to the finished sum (the loop kernel), which is the
+// more exact of the two over a filter's steps (13 points, degree 16, FP32: 8.8e-8 off the
+// 64-bit result against 3.3e-7).
+
+#include "fe_common.cuh"
+
+#include <algorithm>
+#include <vector>
+
+namespace fe {
+namespace {
+
+template <typename T, int VEC>
+struct __align__(VEC * sizeof(T)) Lane {
+  T v[VEC];
+};
+template <typename T, int VEC>
+struct LaneRaw;
+template <> struct LaneRaw<float, 4> { using type = float4; };
+template <> struct LaneRaw<float, 2> { using type = float2; };
+template <> struct LaneRaw<float, 1> { using type = float; };
+template <> struct LaneRaw<double, 2> { using type = double2; };
+template <> struct LaneRaw<double, 1> { using type = double; };
+
+template <typename T>
+struct RowsParams {
+  const int32_t* rowptr;
+  const int32_t* colind;
+  const T* vals;
+  const T* X;
+  T* Y;
+  const T* Z;
+  const T* R;
+  const T* delta;
+  int ldx, ldy, ldz, ldr;  // bytes from row to row
+  int nrows, last_x;       // rows; the last row of X
+  int ncols, pc, panels;   // columns of the block and of a panel, panels
+  int lbx;                 // log2 of a brick's rows along a line
+  int s1, s2;              // rows from line to line, from plane to plane
+  int lines;               // lines of a plane
+  int nx, ny, bz;          // bricks along a line and across a plane, planes of a brick
+  T alpha, gamma, beta;
+  int use_gamma, use_beta;
+};
+
+template <typename T, int VEC>
+__device__ __forceinline__ Lane<T, VEC> load_ro(const T* p) {
+  using R = typename LaneRaw<T, VEC>::type;
+  return __builtin_bit_cast(Lane<T, VEC>, __ldg(reinterpret_cast<const R*>(p)));
+}
+
+constexpr int kRowsThreads = 256;
+
+// G lanes a row, CPL vectors of VEC values a lane, up to M G entries a row, KC neighbours in
+// flight. FOLD: alpha and gamma in the coefficients. TAIL: the columns end inside a vector.
+// CORR: + delta[j] R[row, j].
+template <typename T, int VEC, int G, int CPL, int M, int KC, bool FOLD, bool TAIL, bool CORR>
+__global__ void __launch_bounds__(kRowsThreads, 4)
+spmm_rows_kernel(const __grid_constant__ RowsParams<T> P) {
+  using V = Lane<T, VEC>;
+  constexpr unsigned kFull = 0xffffffffu;
+  constexpr int NG = kRowsThreads / G;
+  const int lane = threadIdx.x & 31;
+  const int gl = threadIdx.x % G;
+  const int grp = threadIdx.x / G;
+  const int panel = blockIdx.x % P.panels;  // panels side by side: whole rows from DRAM
+  const int brick = blockIdx.x / P.panels;
+  const int bx = brick % P.nx, byz = brick / P.nx;
+  const int by = byz % P.ny, bz = byz / P.ny;
+  const int x = (bx << P.lbx) + (grp & ((1 << P.lbx) - 1));
+  const int y = by * (NG >> P.lbx) + (grp >> P.lbx);
+  const int c0 = panel * P.pc;
+  const int nvec = (min(P.pc, P.ncols - c0) + VEC - 1) / VEC;
+  bool act[CPL];
+#pragma unroll
+  for (int q = 0; q < CPL; ++q) act[q] = gl + q * G < nvec;
+  // idle lanes read their group's first vector and store nothing
+  int col[CPL];
+#pragma unroll
+  for (int q = 0; q < CPL; ++q) col[q] = c0 + (act[q] ? (gl + q * G) * VEC : 0);
+  // A last vector that reaches past the block's columns stays inside the row pitch, except
+  // in the last row, whose padding may not be there: read by elements.
+  bool over = false;
+  if constexpr (TAIL) {
+#pragma unroll
+    for (int q = 0; q < CPL; ++q) over |= col[q] + VEC > P.ncols;
+  }
+  const int last_x = over ? P.last_x : -1, last_z = over ? P.nrows - 1 : -2;
+  const char* xp[CPL];
+  const char* zp[CPL];
+  char* yp[CPL];
+#pragma unroll
+  for (int q = 0; q < CPL; ++q) {
+    xp[q] = reinterpret_cast<const char*>(P.X + col[q]);
+    zp[q] = reinterpret_cast<const char*>(P.Z + col[q]);
+    yp[q] = reinterpret_cast<char*>(P.Y + col[q]);
+  }
+  auto at = [](const char* p, int row, int pitch) {
+    return p + static_cast<int64_t>(row) * pitch;
+  };
+  const unsigned mine = G == 32 ? kFull : ((1u << (G & 31)) - 1u) << (lane - gl);
+  const bool in = x < P.s1 && y < P.lines;
+  int64_t r64 = x + static_cast<int64_t>(P.s1) * y + static_cast<int64_t>(P.s2) * bz * P.bz;
+  int row = in && r64 < P.nrows ? static_cast<int>(r64) : -1;
+  int zi = 0;
+  auto next_of = [&](int r) {
+    const unsigned n = static_cast<unsigned>(r) + static_cast<unsigned>(P.s2);
+    return r >= 0 && n < static_cast<unsigned>(P.nrows) ? static_cast<int>(n) : -1;
+  };
+  int s = 0, e = 0;
+  if (row >= 0) {
+    s = __ldg(P.rowptr + row);
+    e = __ldg(P.rowptr + row + 1);
+  }
+  int c[M];
+  T w[M];
+#pragma unroll
+  for (int m = 0; m < M; ++m) {
+    c[m] = -2;
+    w[m] = T(0);
+    if (s + m * G + gl < e) {
+      c[m] = __ldg(P.colind + s + m * G + gl);
+      w[m] = __ldg(P.vals + s + m * G + gl);
+    }
+  }
+  int nrow = P.bz > 1 ? next_of(row) : -1;
+  int ns = 0, ne = 0;
+  if (nrow >= 0) {
+    ns = __ldg(P.rowptr + nrow);
+    ne = __ldg(P.rowptr + nrow + 1);
+  }
+  while (true) {
+    const int cnt = e - s;
+    V z[CPL];
+    if (P.use_beta && row >= 0) {
+#pragma unroll
+      for (int q = 0; q < CPL; ++q) {
+        const T* p = reinterpret_cast<const T*>(at(zp[q], row, P.ldz));
+        if (TAIL && row == last_z) {
+#pragma unroll
+          for (int f = 0; f < VEC; ++f) z[q].v[f] = col[q] + f < P.ncols ? p[f] : T(0);
+        } else {
+          z[q] = *reinterpret_cast<const V*>(p);
+        }
+      }
+    }
+    bool self = false;
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+      if (!FOLD) break;
+      w[m] = P.alpha * w[m];
+      if (P.use_gamma) {
+        const bool own = c[m] == row;  // lanes past the row's entries hold column -2
+        self |= own;
+        if (own) w[m] += P.gamma;
+      }
+    }
+    V acc[CPL];
+#pragma unroll
+    for (int q = 0; q < CPL; ++q)
+#pragma unroll
+      for (int f = 0; f < VEC; ++f) acc[q].v[f] = T(0);
+    int cn[M];
+    T wn[M];
+    int nrow2 = -1, ns2 = 0, ne2 = 0;
+    auto prefetch = [&] {
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        cn[m] = -2;
+        wn[m] = T(0);
+        if (ns + m * G + gl < ne) {
+          cn[m] = __ldg(P.colind + ns + m * G + gl);
+          wn[m] = __ldg(P.vals + ns + m * G + gl);
+        }
+      }
+      nrow2 = zi + 2 < P.bz ? next_of(nrow) : -1;
+      if (nrow2 >= 0) {
+        ns2 = __ldg(P.rowptr + nrow2);
+        ne2 = __ldg(P.rowptr + nrow2 + 1);
+      }
+    };
+    auto fetch = [&](int cj, int q) -> V {
+      const T* p = reinterpret_cast<const T*>(at(xp[q], cj, P.ldx));
+      if constexpr (TAIL) {
+        if (cj == last_x) {
+          V r;
+#pragma unroll
+          for (int f = 0; f < VEC; ++f) r.v[f] = col[q] + f < P.ncols ? __ldg(p + f) : T(0);
+          return r;
+        }
+      }
+      return load_ro<T, VEC>(p);
+    };
+    const int cnt0 = __shfl_sync(kFull, cnt, 0);
+    if (__all_sync(kFull, cnt == cnt0)) {
+      // every row of the warp has as many entries: no lane is held back
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+#pragma unroll
+        for (int j0 = 0; j0 < G; j0 += KC) {
+          const int base = m * G + j0;
+          if (base + KC <= cnt0 && j0 + KC <= G) {
+            V xv[KC][CPL];
+#pragma unroll
+            for (int j = 0; j < KC; ++j) {
+              const int cj = __shfl_sync(kFull, c[m], j0 + j, G);
+#pragma unroll
+              for (int q = 0; q < CPL; ++q) xv[j][q] = fetch(cj, q);
+            }
+            if (base == 0) prefetch();
+#pragma unroll
+            for (int j = 0; j < KC; ++j) {
+              const T wj = __shfl_sync(kFull, w[m], j0 + j, G);
+#pragma unroll
+              for (int q = 0; q < CPL; ++q)
+#pragma unroll
+                for (int f = 0; f < VEC; ++f) acc[q].v[f] = fma(wj, xv[j][q].v[f], acc[q].v[f]);
+            }
+          } else if (base < cnt0) {
+            if (base == 0) prefetch();
+#pragma unroll
+            for (int j = 0; j < KC; ++j) {
+              if (j0 + j < G && base + j < cnt0) {
+                const int cj = __shfl_sync(kFull, c[m], j0 + j, G);
+                const T wj = __shfl_sync(kFull, w[m], j0 + j, G);
+#pragma unroll
+                for (int q = 0; q < CPL; ++q) {
+                  const V xv = fetch(cj, q);
+#pragma unroll
+                  for (int f = 0; f < VEC; ++f) acc[q].v[f] = fma(wj, xv.v[f], acc[q].v[f]);
+                }
+              }
+            }
+          }
+        }
+      }
+      if (cnt0 == 0) prefetch();
+    } else {
+      prefetch();
+      int most = cnt;
+#pragma unroll
+      for (int o = 16; o >= G; o >>= 1) most = max(most, __shfl_xor_sync(kFull, most, o));
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        for (int j = 0; j < G; ++j) {
+          if (m * G + j >= most) break;
+          const int cj = __shfl_sync(kFull, c[m], j, G);
+          const T wj = __shfl_sync(kFull, w[m], j, G);
+          if (m * G + j < cnt) {
+#pragma unroll
+            for (int q = 0; q < CPL; ++q) {
+              const V xv = fetch(cj, q);
+#pragma unroll
+              for (int f = 0; f < VEC; ++f) acc[q].v[f] = fma(wj, xv.v[f], acc[q].v[f]);
+            }
+          }
+        }
+      }
+    }
+    if (FOLD && P.use_gamma) {
+      const unsigned found = __ballot_sync(kFull, self);
+      if (row >= 0 && !(found & mine)) {
+#pragma unroll
+        for (int q = 0; q < CPL; ++q) {
+          const V xv = fetch(row, q);
+#pragma unroll
+          for (int f = 0; f < VEC; ++f) acc[q].v[f] = fma(P.gamma, xv.v[f], acc[q].v[f]);
+        }
+      }
+    }
+    if (row >= 0) {
+#pragma unroll
+      for (int q = 0; q < CPL; ++q) {
+        V out = acc[q];
+        if constexpr (!FOLD) {
+#pragma unroll
+          for (int f = 0; f < VEC; ++f) out.v[f] = P.alpha * out.v[f];
+          if (P.use_gamma) {  // the row of X is in L1
+            const V xv = fetch(row, q);
+#pragma unroll
+            for (int f = 0; f < VEC; ++f) out.v[f] = fma(P.gamma, xv.v[f], out.v[f]);
+          }
+        }
+        if (P.use_beta) {
+#pragma unroll
+          for (int f = 0; f < VEC; ++f) out.v[f] = fma(P.beta, z[q].v[f], out.v[f]);
+        }
+        if (act[q]) {
+          if constexpr (CORR) {
+            const V rv = *reinterpret_cast<const V*>(
+                at(reinterpret_cast<const char*>(P.R + col[q]), row, P.ldr));
+#pragma unroll
+            for (int f = 0; f < VEC; ++f)
+              out.v[f] = fma(__ldg(P.delta + col[q] + f), rv.v[f], out.v[f]);
+          }
+          T* yr = reinterpret_cast<T*>(yp[q] + static_cast<int64_t>(row) * P.ldy);
+          if (TAIL && col[q] + VEC > P.ncols) {
+#pragma unroll
+            for (int f = 0; f < VEC; ++f)
+              if (col[q] + f < P.ncols) yr[f] = out.v[f];
+          } else {
+            *reinterpret_cast<V*>(yr) = out;
+          }
+        }
+      }
+    }
+    if (++zi >= P.bz || !__any_sync(kFull, nrow >= 0)) break;
+    row = nrow;
+    nrow = nrow2;
+    s = ns;
+    e = ne;
+    ns = ns2;
+    ne = ne2;
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+      c[m] = cn[m];
+      w[m] = wn[m];
+    }
+  }
+}
+
+template <typename T, int VEC, int G, int CPL, int M, int KC, bool FOLD, bool CORR>
+void launch(RowsParams<T> P, int64_t rows, bool tail, cudaStream_t s) {
+  constexpr int NG = kRowsThreads / G;
+  // Bricks of 4 lines; without a grid the "planes" are runs of NG consecutive rows.
+  int by = NG / 4;
+  if (P.s1 == 0) {
+    P.s1 = P.s2 = NG;
+    P.lines = 1;
+    by = 1;
+  } else if (P.s2 == 0) {  // a grid of lines only: sweep down groups of `by` lines
+    P.lines = by;
+    P.s2 = P.s1 * by;
+  } else {
+    P.lines = P.s2 / P.s1;
+  }
+  P.lbx = 0;
+  while ((by << P.lbx) < NG) ++P.lbx;
+  P.nx = (P.s1 + (1 << P.lbx) - 1) >> P.lbx;
+  P.ny = (P.lines + by - 1) / by;
+  const int64_t planes = (rows + P.s2 - 1) / P.s2;
+  const int64_t columns = static_cast<int64_t>(P.nx) * P.ny * P.panels;
+  // Deep bricks re-read fewer planes, as long as every SM still gets about three rounds of
+  // its four CTAs.
+  P.bz = 16;
+  while (P.bz > 1 && columns * ((planes + P.bz - 1) / P.bz) < int64_t(12) * num_sms()) P.bz /= 2;
+  const int64_t grid = columns * ((planes + P.bz - 1) / P.bz);
+  FE_REQUIRE(grid <= 0x7fffffffLL, "csr_spmm: too many rows for one launch");
+  if (VEC > 1 && tail)
+    spmm_rows_kernel<T, VEC, G, CPL, M, KC, FOLD, (VEC > 1), CORR>
+        <<<static_cast<unsigned>(grid), kRowsThreads, 0, s>>>(P);
+  else
+    spmm_rows_kernel<T, VEC, G, CPL, M, KC, FOLD, false, CORR>
+        <<<static_cast<unsigned>(grid), kRowsThreads, 0, s>>>(P);
+  check_launch("spmm_rows_kernel");
+}
+
+// Line and plane strides of the grid behind a row's column offsets: runs of offsets that
+// differ by 1 are one neighbour along the line (s1: the centre of the first run past the
+// line's own neighbours), runs of those that differ by up to two lines one plane.
+void grid_strides(const int32_t* cols, int count, int64_t row, int64_t rows, int* s1, int* s2) {
+  *s1 = *s2 = 0;
+  std::vector<int> d;
+  for (int i = 0; i < count; ++i)
+    if (cols[i] > row) d.push_back(static_cast<int>(cols[i] - row));
+  std::sort(d.begin(), d.end());
+  size_t i = 0;
+  while (i < d.size() && d[i] < 4) ++i;
+  if (i == d.size()) return;
+  size_t j = i;
+  while (j + 1 < d.size() && d[j + 1] - d[j] <= 1) ++j;
+  const int line = (d[i] + d[j]) / 2;
+  if (line < 4 || line > rows / 2) return;
+  *s1 = line;
+  i = j + 1;
+  while (i < d.size() && d[i] <= 3 * line) ++i;
+  if (i == d.size()) return;
+  j = i;
+  while (j + 1 < d.size() && d[j + 1] - d[j] <= 2 * line + 2) ++j;
+  const int plane = (d[i] + d[j]) / 2;
+  if (plane % line == 0 && plane <= rows / 2) *s2 = plane;
+}
+
+}  // namespace
+
+// Looks at the longest of a few rows in the middle of the operator (a heuristic: the result
+// only orders the work).
+void csr_find_grid(Csr& A, const int32_t* rowptr, const int32_t* colind, int64_t row0,
+                   int64_t count) {
+  A.grid_s1 = A.grid_s2 = 0;
+  int64_t best = -1;
+  for (int64_t i = 0; i < count; ++i)
+    if (best < 0 || rowptr[i + 1] - rowptr[i] > rowptr[best + 1] - rowptr[best]) best = i;
+  if (best < 0) return;
+  grid_strides(colind + (rowptr[best] - rowptr[0]), rowptr[best + 1] - rowptr[best], row0 + best,
+               A.rows, &A.grid_s1, &A.grid_s2);
+}
+
+// The same for an operator whose arrays are on the device.
+void csr_find_grid_device(Csr& A) {
+  A.grid_s1 = A.grid_s2 = 0;
+  if (A.rows < 64 || A.nnz == 0) return;
+  const int64_t row0 = A.rows / 2 - 16, count = 32;
+  std::vector<int32_t> rp(count + 1);
+  FE_CHECK_CUDA(cudaMemcpy(rp.data(), A.rowptr + row0, rp.size() * sizeof(int32_t),
+                           cudaMemcpyDeviceToHost));
+  std::vector<int32_t> ci(std::max(1, rp[count] - rp[0]));
+  if (rp[count] > rp[0])
+    FE_CHECK_CUDA(cudaMemcpy(ci.data(), A.colind + rp[0], (rp[count] - rp[0]) * sizeof(int32_t),
+                             cudaMemcpyDeviceToHost));
+  csr_find_grid(A, rp.data(), ci.data(), row0, count);
+}
+
+template <typename T>
+bool csr_spmm_rows(const Csr& A, const T* X, int64_t ldx, T* Y, int64_t ldy, const T* Z,
+                   int64_t ldz, const T* R, int64_t ldr, const T* delta, int64_t ncols,
+                   double alpha, double gamma, double beta, cudaStream_t s) {
+  constexpr int V16 = 16 / sizeof(T);
+  const bool ub = beta != 0.0;
+  const int k = static_cast<int>(std::min<int64_t>(A.max_row_nnz, 64));
+  const int64_t bytes = ncols * static_cast<int64_t>(sizeof(T));
+  const int64_t far = std::max(std::max(ldx, ldy), std::max(ub ? ldz : 0, R ? ldr : 0));
+  // A vector's columns fit the wide row kernel better than panels without a grid's reuse:
+  // 320 FP32 columns take 1.91 ms there and 2.35 ms here (128^3); 160 columns 714 against
+  // 475 us (96^3). Blocks of up to four vectors keep the loop kernel's smaller groups.
+  if (k < 1 || k > 32 || bytes <= 64 || far * static_cast<int64_t>(sizeof(T)) > 0x7fffffffLL)
+    return false;
+  if (A.grid_s1 == 0 && bytes > 1024) return false;
+  auto multiple = [&](size_t b) {
+    auto ok = [b](const void* p, int64_t ld) {
+      return reinterpret_cast<uintptr_t>(p) % b == 0 && (ld * sizeof(T)) % b == 0;
+    };
+    return ok(X, ldx) && ok(Y, ldy) && (!ub || ok(Z, ldz)) && (!R || ok(R, ldr));
+  };
+  const int vec = multiple(16) ? V16 : sizeof(T) == 4 && multiple(8) ? 2 : 1;
+  if (R && (vec != V16 || ncols % V16 != 0)) return false;
+  RowsParams<T> P{};
+  P.rowptr = A.rowptr;
+  P.colind = A.colind;
+  if constexpr (sizeof(T) == 8) P.vals = A.val64; else P.vals = A.val32;
+  P.X = X;
+  P.Y = Y;
+  P.Z = Z;
+  P.R = R;
+  P.delta = delta;
+  P.ldx = static_cast<int>(ldx * sizeof(T));
+  P.ldy = static_cast<int>(ldy * sizeof(T));
+  P.ldz = static_cast<int>(ldz * sizeof(T));
+  P.ldr = static_cast<int>(ldr * sizeof(T));
+  P.nrows = static_cast<int>(A.rows);
+  P.last_x = static_cast<int>(A.cols) - 1;
+  P.ncols = static_cast<int>(ncols);
+  P.s1 = A.grid_s1;
+  P.s2 = A.grid_s2;
+  P.alpha = static_cast<T>(alpha);
+  P.gamma = static_cast<T>(gamma);
+  P.beta = static_cast<T>(beta);
+  P.use_gamma = gamma != 0.0 ? 1 : 0;
+  P.use_beta = ub ? 1 : 0;
+  // as the row kernel of spmm.cu would take it: short rows, 32 or more 8-byte vectors
+  const bool fold = k <= 7 && vec * sizeof(T) >= 8 && bytes % 8 == 0 && bytes >= 256;
+  const bool tail = ncols % vec != 0;
+  const int nvec = static_cast<int>((ncols + vec - 1) / vec);
+  auto panels = [&](int cap) {
+    P.panels = (nvec + cap - 1) / cap;
+    P.pc = (nvec + P.panels - 1) / P.panels * vec;
+  };
+#define FE_ROWS_F(V_, G_, C_, M_, K_, FOLD_, CORR_)                 \
+  do {                                                              \
+    panels(G_ * C_);                                                \
+    launch<T, V_, G_, C_, M_, K_, FOLD_, CORR_>(P, A.rows, tail, s); \
+    return true;                                                    \
+  } while (0)
+#define FE_ROWS(V_, G_, C_, M_, K_, CORR_)                      \
+  do {                                                          \
+    if (fold) FE_ROWS_F(V_, G_, C_, M_, K_, true, CORR_);       \
+    FE_ROWS_F(V_, G_, C_, M_, K_, false, CORR_);                \
+  } while (0)
+  if (vec == V16) {
+    // 128-byte panels where 256-byte ones would leave more than a tenth more lanes idle
+    // (160 FP32 columns: 5 full panels of 128 bytes, 422 us, or 3 of 256, 433 us; 96^3).
+    const int lanes16 = (nvec + 15) / 16 * 16, lanes8 = (nvec + 7) / 8 * 8;
+    const bool narrow = k <= 16 && lanes8 * 10 < lanes16 * 9;
+    if constexpr (sizeof(T) == 4) {
+      if (R) {
+        if (narrow && k <= 8) FE_ROWS(V16, 8, 1, 1, 7, true);
+        if (narrow) FE_ROWS_F(V16, 8, 1, 2, 4, false, true);
+        if (k <= 8) FE_ROWS(V16, 16, 1, 1, 7, true);
+        if (k <= 16) FE_ROWS_F(V16, 16, 1, 1, 4, false, true);
+        FE_ROWS_F(V16, 16, 1, 2, 8, false, true);
+      }
+    }
+    if (narrow && k <= 8) FE_ROWS(V16, 8, 1, 1, 7, false);
+    if (narrow) FE_ROWS_F(V16, 8, 1, 2, 4, false, false);
+    if (k <= 8) FE_ROWS(V16, 16, 1, 1, 7, false);
+    if (k <= 16) FE_ROWS_F(V16, 16, 1, 1, 4, false, false);
+    FE_ROWS_F(V16, 16, 1, 2, 8, false, false);
+  }
+  if constexpr (sizeof(T) == 4) {
+    if (vec == 2) {
+      if (k <= 16) FE_ROWS(2, 16, 2, 1, 4, false);
+      FE_ROWS_F(2, 16, 2, 2, 4, false, false);
+    }
+  }
+  // rows that start at any element: up to three elements a lane
+  if (nvec <= 16 && k <= 16) FE_ROWS_F(1, 16, 1, 1, 4, false, false);
+  if (nvec <= 32 && k <= 16) FE_ROWS(1, 16, 2, 1, 4, false);
+  if (k <= 16) FE_ROWS(1, 16, 3, 1, 4, false);
+  FE_ROWS_F(1, 16, 3, 2, 4, false, false);
+#undef FE_ROWS_F
+#undef FE_ROWS
+}
+template bool csr_spmm_rows<float>(const Csr&, const float*, int64_t, float*, int64_t,
+                                   const float*, int64_t, const float*, int64_t, const float*,
+                                   int64_t, double, double, double, cudaStream_t);
+template bool csr_spmm_rows<double>(const Csr&, const double*, int64_t, double*, int64_t,
+                                    const double*, int64_t, const double*, int64_t,
+                                    const double*, int64_t, double, double, double,
+                                    cudaStream_t);
+
+}  // namespace fe

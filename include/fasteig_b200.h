@@ -202,8 +202,9 @@ int fe_device_status(int32_t* status, int32_t clear);
 int fe_selftest_wait_timeout(int64_t limit_cycles, int32_t code, void* stream);
 /* SpMM kernel selection for all later calls in the process (the numerics are
  * the same; the choice only changes the memory schedule): 0 = default
- * (row-batched register kernel for slabs of >= 32 128-bit vectors and rows of
- * <= 7 nonzeros, else the loop kernel), 1 = loop kernel, 2 = bulk-copy
+ * (several rows to a warp for rows of <= 32 nonzeros, in bricks of the operator's
+ * grid; without a grid and with more than 1 KiB of a row the row-batched register
+ * kernel for rows of <= 7 nonzeros; else the loop kernel), 1 = loop kernel, 2 = bulk-copy
  * pipelined kernel where it applies, 3 = row-batched kernel with narrower
  * column panels, 4 = mode 0 with each warp's next Z row prefetched into L2,
  * 5 = row-batched kernel with 16-byte lanes and up to 3 per lane, 6 = row-batched
