@@ -208,68 +208,117 @@ rotate_kernel(const T* __restrict__ X, int64_t ldx, const double* __restrict__ C
 }
 
 // -------------------------------------------------- Residual and norms ----
-constexpr int kNormCols = 32;       // columns per CTA (one per lane)
-constexpr int kNormTargetChunks = 256;
+// Three streams (AX, M X, R) at two rounded operations a value: DRAM bound. One CTA per SM
+// takes a run of whole rows; its threads are dealt over the row's 16-byte vectors and over
+// rows, four rows of a thread in flight, so that every row is read in full lines and the
+// SM has up to 190 KB under way. (One warp per 32 columns, a value a lane and a row at a
+// time, took 477 us a call for 512,000 x 96 FP64 with B and R, 2.5 TB/s; this takes 223 us,
+// 5.3 TB/s.)
+constexpr int kNormThreads = 1024;
+constexpr int kNormMaxVecs = 512;  // vectors of a row that one CTA takes
+constexpr int kNormMaxChunks = 148;
+constexpr int kNormRows = 4;  // rows of a thread in flight
 
-// R = AX - lambda * MX, per-column sums of squares of R and MX (FP64), per chunk.
-template <typename T>
-__global__ void __launch_bounds__(256)
+template <typename T, int VEC>
+struct __align__(VEC * sizeof(T)) NormVec {
+  T v[VEC];
+};
+
+// R = AX - lambda * MX, per-column sums of squares of R and MX (FP64), per chunk of rows.
+// MODE 0: norms of X (of BX when given) only; 1: residual; 2: B-norms sqrt(x . Bx) of the
+// columns of X (BX required).
+template <typename T, int VEC, int MODE>
+__global__ void __launch_bounds__(kNormThreads)
 residual_partial_kernel(const T* __restrict__ AX, const T* __restrict__ X,
                         const T* __restrict__ BX, int64_t ld, int64_t n, int m,
                         const double* __restrict__ lambda, T* __restrict__ R, int64_t ldr,
-                        int64_t rows_per_chunk, double* __restrict__ partial, int mode) {
-  // mode 0: norms of X (of BX when given) only; mode 1: residual; mode 2: B-norms
-  // sqrt(x . Bx) of the columns of X (BX required).
-  __shared__ double red[2][8][kNormCols];
-  const int lane = threadIdx.x % 32;
-  const int warp = threadIdx.x / 32;
-  const int j = blockIdx.x * kNormCols + lane;
+                        int64_t rows_per_chunk, double* __restrict__ partial) {
+  using V = NormVec<T, VEC>;
+  extern __shared__ double red[];  // [row share][2][columns of this CTA]
+  const int col0 = blockIdx.x * kNormMaxVecs * VEC;
+  const int cols = min(m - col0, kNormMaxVecs * VEC);
+  const int vecs = cols / VEC;  // exact: VEC > 1 only where VEC divides m
+  const int shares = kNormThreads / vecs;
+  const int share = threadIdx.x / vecs;
+  const int j = col0 + (threadIdx.x - share * vecs) * VEC;
   const int64_t r_begin = static_cast<int64_t>(blockIdx.y) * rows_per_chunk;
   const int64_t r_end = min(n, r_begin + rows_per_chunk);
-  double sr = 0.0, sx = 0.0;
-  if (j < m) {
-    const double lam = mode == 1 ? lambda[j] : 0.0;
+  double sr[VEC], sx[VEC], lam[VEC];
+#pragma unroll
+  for (int e = 0; e < VEC; ++e) {
+    sr[e] = sx[e] = 0.0;
+    lam[e] = MODE == 1 && share < shares ? lambda[j + e] : 0.0;
+  }
+  if (share < shares) {
     const T* M = BX ? BX : X;
-    for (int64_t r = r_begin + warp; r < r_end; r += 8) {
-      const double mx = static_cast<double>(M[r * ld + j]);
-      if (mode == 2) {  // B-inner products x . (Bx)
-        sx = fma(static_cast<double>(X[r * ld + j]), mx, sx);
-        continue;
+    for (int64_t r0 = r_begin + share; r0 < r_end; r0 += kNormRows * shares) {
+      V mx[kNormRows], ax[kNormRows];
+#pragma unroll
+      for (int u = 0; u < kNormRows; ++u) {
+        const int64_t r = r0 + u * shares;
+        if (r < r_end) {
+          mx[u] = *reinterpret_cast<const V*>(M + r * ld + j);
+          if (MODE == 1) ax[u] = *reinterpret_cast<const V*>(AX + r * ld + j);
+          if (MODE == 2) ax[u] = *reinterpret_cast<const V*>(X + r * ld + j);
+        }
       }
-      sx = fma(mx, mx, sx);
-      if (mode == 1) {
-        const T rv = static_cast<T>(static_cast<double>(AX[r * ld + j]) - lam * mx);
-        if (R) R[r * ldr + j] = rv;
-        const double rd = static_cast<double>(rv);
-        sr = fma(rd, rd, sr);
+#pragma unroll
+      for (int u = 0; u < kNormRows; ++u) {
+        const int64_t r = r0 + u * shares;
+        if (r < r_end) {
+          V out;
+#pragma unroll
+          for (int e = 0; e < VEC; ++e) {
+            const double x = static_cast<double>(mx[u].v[e]);
+            if (MODE == 2) {  // B-inner products x . (Bx)
+              sx[e] = fma(static_cast<double>(ax[u].v[e]), x, sx[e]);
+              continue;
+            }
+            sx[e] = fma(x, x, sx[e]);
+            if (MODE == 1) {
+              const T rv = static_cast<T>(static_cast<double>(ax[u].v[e]) - lam[e] * x);
+              out.v[e] = rv;
+              const double rd = static_cast<double>(rv);
+              sr[e] = fma(rd, rd, sr[e]);
+            }
+          }
+          if (MODE == 1 && R) *reinterpret_cast<V*>(R + r * ldr + j) = out;
+        }
       }
+    }
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) {
+      red[(2 * share) * cols + j - col0 + e] = sr[e];
+      red[(2 * share + 1) * cols + j - col0 + e] = sx[e];
     }
   }
-  red[0][warp][lane] = sr;
-  red[1][warp][lane] = sx;
   __syncthreads();
-  if (warp == 0 && j < m) {
-    double a = 0.0, b = 0.0;
-    for (int w = 0; w < 8; ++w) {
-      a += red[0][w][lane];
-      b += red[1][w][lane];
-    }
-    double* out = partial + static_cast<int64_t>(blockIdx.y) * 2 * m;
-    out[j] = a;
-    out[m + j] = b;
+  for (int i = threadIdx.x; i < 2 * cols; i += kNormThreads) {
+    double a = 0.0;
+    for (int q = 0; q < shares; ++q) a += red[2 * q * cols + i];
+    const int half = i / cols;
+    partial[static_cast<int64_t>(blockIdx.y) * 2 * m + half * m + col0 + (i - half * cols)] = a;
   }
 }
 
+// A warp per column: the chunks' sums in a fixed order (lane, then a fixed tree).
 __global__ void residual_finish_kernel(const double* __restrict__ partial, int chunks, int m,
                                        const double* __restrict__ lambda, double* rnorm,
                                        double* xnorm, double* rel, int mode) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = (blockIdx.x * blockDim.x + threadIdx.x) / 32;
+  const int lane = threadIdx.x & 31;
   if (j >= m) return;
   double a = 0.0, b = 0.0;
-  for (int c = 0; c < chunks; ++c) {
+  for (int c = lane; c < chunks; c += 32) {
     a += partial[static_cast<int64_t>(c) * 2 * m + j];
     b += partial[static_cast<int64_t>(c) * 2 * m + m + j];
   }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_down_sync(0xffffffffu, a, o);
+    b += __shfl_down_sync(0xffffffffu, b, o);
+  }
+  if (lane != 0) return;
   const double rn = sqrt(a);
   const double xn = sqrt(fmax(b, 0.0));
   if (mode != 1) {
@@ -285,22 +334,43 @@ __global__ void residual_finish_kernel(const double* __restrict__ partial, int c
 }
 
 struct NormPlan {
-  int col_blocks, chunks;
+  int chunks;
   int64_t rows_per_chunk;
   size_t bytes;
 };
 
+// Row chunks: one CTA per SM, of 64 rows at least.
 NormPlan norm_plan(int64_t n, int64_t m) {
   NormPlan p{};
-  p.col_blocks = static_cast<int>((m + kNormCols - 1) / kNormCols);
-  int64_t chunks = std::max<int64_t>(1, kNormTargetChunks / std::max(1, p.col_blocks));
-  chunks = std::max<int64_t>(1, std::min<int64_t>(chunks, (n + 63) / 64));
-  int64_t rpc = (n + chunks - 1) / chunks;
-  p.rows_per_chunk = std::max<int64_t>(1, rpc);
-  p.chunks = static_cast<int>((n + p.rows_per_chunk - 1) / p.rows_per_chunk);
-  if (p.chunks < 1) p.chunks = 1;
+  const int64_t chunks = std::max<int64_t>(1, std::min<int64_t>(kNormMaxChunks, (n + 63) / 64));
+  p.rows_per_chunk = std::max<int64_t>(1, (n + chunks - 1) / chunks);
+  p.chunks = static_cast<int>(std::max<int64_t>(1, (n + p.rows_per_chunk - 1) / p.rows_per_chunk));
   p.bytes = static_cast<size_t>(p.chunks) * 2 * std::max<int64_t>(m, 1) * sizeof(double);
   return p;
+}
+
+template <typename T, int VEC, int MODE>
+void launch_residual(const T* AX, const T* X, const T* BX, int64_t ld, int64_t n, int m,
+                     const double* lambda, T* R, int64_t ldr, const NormPlan& p, double* partial,
+                     cudaStream_t s) {
+  auto kern = residual_partial_kernel<T, VEC, MODE>;
+  // shares x columns of a CTA: at most kNormThreads x VEC, whatever its columns
+  const size_t smem = static_cast<size_t>(2) * kNormThreads * VEC * sizeof(double);
+  FE_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     static_cast<int>(smem)));
+  const int blocks = (m + kNormMaxVecs * VEC - 1) / (kNormMaxVecs * VEC);
+  kern<<<dim3(blocks, p.chunks), kNormThreads, smem, s>>>(AX, X, BX, ld, n, m, lambda, R, ldr,
+                                                          p.rows_per_chunk, partial);
+  check_launch("residual_partial_kernel");
+}
+
+template <typename T, int VEC>
+void launch_residual(const T* AX, const T* X, const T* BX, int64_t ld, int64_t n, int m,
+                     const double* lambda, T* R, int64_t ldr, const NormPlan& p, double* partial,
+                     int mode, cudaStream_t s) {
+  if (mode == 1) launch_residual<T, VEC, 1>(AX, X, BX, ld, n, m, lambda, R, ldr, p, partial, s);
+  else if (mode == 2) launch_residual<T, VEC, 2>(AX, X, BX, ld, n, m, lambda, R, ldr, p, partial, s);
+  else launch_residual<T, VEC, 0>(AX, X, BX, ld, n, m, lambda, R, ldr, p, partial, s);
 }
 
 template <typename S, typename D>
@@ -616,7 +686,7 @@ template void rotate<float>(const float*, int64_t, const double*, int64_t, float
 // target count nor one per 64 rows).
 size_t residual_workspace_bytes(int64_t n, int64_t m) {
   if (n <= 0 || m <= 0) return 0;
-  const int64_t chunks = std::min<int64_t>(kNormTargetChunks, (n + 63) / 64 + 1);
+  const int64_t chunks = std::min<int64_t>(256, (n + 63) / 64 + 1);
   return static_cast<size_t>(chunks) * 2 * m * sizeof(double);
 }
 
@@ -631,19 +701,24 @@ void residual_norms(const T* AX, const T* X, const T* BX, int64_t ld, int64_t n,
   if (mode == 1) FE_REQUIRE(AX && lambda, "residual_norms: missing AX or lambda");
   if (mode == 2) FE_REQUIRE(BX, "residual_norms: B-norms need BX");
   if (R) FE_REQUIRE(ldr >= m, "residual_norms: invalid R leading dimension");
-  FE_REQUIRE(m <= 65535LL * kNormCols, "residual_norms: too many columns");
+  FE_REQUIRE(m <= 65535LL * 32, "residual_norms: too many columns");
   const NormPlan p = norm_plan(std::max<int64_t>(n, 1), m);
   FE_REQUIRE(ws && ws_bytes >= p.bytes, "residual_norms: workspace too small");
   if (n == 0) {
     FE_CHECK_CUDA(cudaMemsetAsync(ws, 0, p.bytes, s));
   } else {
-    dim3 grid(p.col_blocks, p.chunks);
-    residual_partial_kernel<T><<<grid, 256, 0, s>>>(AX, X, BX, ld, n, static_cast<int>(m), lambda,
-                                                    R, ldr, p.rows_per_chunk,
-                                                    static_cast<double*>(ws), mode);
-    check_launch("residual_partial_kernel");
+    constexpr int V16 = 16 / sizeof(T);
+    auto rows16 = [](const T* q, int64_t pitch) { return !q || (aligned16(q) && pitch % V16 == 0); };
+    const bool vec = m % V16 == 0 && rows16(AX, ld) && rows16(X, ld) && rows16(BX, ld) &&
+                     rows16(R, ldr);
+    double* partial = static_cast<double*>(ws);
+    const int cols = static_cast<int>(m);
+    if (vec)
+      launch_residual<T, V16>(AX, X, BX, ld, n, cols, lambda, R, ldr, p, partial, mode, s);
+    else
+      launch_residual<T, 1>(AX, X, BX, ld, n, cols, lambda, R, ldr, p, partial, mode, s);
   }
-  residual_finish_kernel<<<static_cast<unsigned>((m + 127) / 128), 128, 0, s>>>(
+  residual_finish_kernel<<<static_cast<unsigned>((m + 7) / 8), 256, 0, s>>>(
       static_cast<const double*>(ws), n == 0 ? 1 : p.chunks, static_cast<int>(m), lambda, rnorm,
       xnorm, rel, mode);
   check_launch("residual_finish_kernel");
