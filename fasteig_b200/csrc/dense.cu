@@ -186,153 +186,228 @@ int num_sms() {
 
 namespace {
 
-// Right-looking unblocked Cholesky in one CTA. G is column-major (ldg); on
-// return its upper triangle holds R (G = R^T R) and the strict lower part is 0.
-__global__ void __launch_bounds__(1024)
-potrf_upper_kernel(double* G, int k, int64_t ldg, int32_t* info) {
-  __shared__ double inv_pivot;
-  __shared__ int failed;
-  if (threadIdx.x == 0) failed = 0;
-  __syncthreads();
-  for (int j = 0; j < k; ++j) {
-    if (threadIdx.x == 0) {
-      const double d = G[static_cast<int64_t>(j) * ldg + j];
-      if (!(d > 0.0) || !isfinite(d)) {
-        failed = j + 1;
-      } else {
-        const double r = sqrt(d);
-        G[static_cast<int64_t>(j) * ldg + j] = r;
-        inv_pivot = 1.0 / r;
-      }
-    }
-    __syncthreads();
-    if (failed) break;
-    // Row j of R: R[j][c] = G[j][c] / r_jj for c > j.
-    for (int c = j + 1 + threadIdx.x; c < k; c += blockDim.x) {
-      G[static_cast<int64_t>(c) * ldg + j] *= inv_pivot;
-    }
-    __syncthreads();
-    // Trailing update of the upper triangle: G[a][c] -= R[j][a] R[j][c], j < a <= c.
-    const int t = k - j - 1;
-    const int64_t count = static_cast<int64_t>(t) * (t + 1) / 2;
-    for (int64_t idx = threadIdx.x; idx < count; idx += blockDim.x) {
-      // Map idx to (a, c) with a <= c in the trailing t-by-t triangle, column-wise:
-      // column cc holds rows 0..cc, offset cc*(cc+1)/2.
-      int cc = static_cast<int>((sqrt(8.0 * static_cast<double>(idx) + 1.0) - 1.0) * 0.5);
-      while (static_cast<int64_t>(cc + 1) * (cc + 2) / 2 <= idx) ++cc;
-      while (static_cast<int64_t>(cc) * (cc + 1) / 2 > idx) --cc;
-      const int aa = static_cast<int>(idx - static_cast<int64_t>(cc) * (cc + 1) / 2);
-      const int a = j + 1 + aa;
-      const int c = j + 1 + cc;
-      G[static_cast<int64_t>(c) * ldg + a] -=
-          G[static_cast<int64_t>(a) * ldg + j] * G[static_cast<int64_t>(c) * ldg + j];
-    }
-    __syncthreads();
-  }
-  // Zero the strict lower triangle.
-  for (int64_t idx = threadIdx.x; idx < static_cast<int64_t>(k) * k; idx += blockDim.x) {
-    const int r = static_cast<int>(idx % k);
-    const int c = static_cast<int>(idx / k);
-    if (r > c) G[static_cast<int64_t>(c) * ldg + r] = 0.0;
-  }
-  if (threadIdx.x == 0 && info) *info = failed;
+// Blocked left-looking Cholesky (upper, G = R^T R) in one CTA, 32 rows of R at a time. For
+// block row J (rows j0..j0+31):
+//   1. G[J, c] -= R[0:j0, J]^T R[0:j0, c], c >= j0, on the FP64 tensor cores: R[0:j0, J]
+//      is staged in shared memory, each warp takes 8 columns and streams their finished
+//      entries from L2 (every one is read once per block row).
+//   2. One warp factors the diagonal block in registers, a lane per column; a finished row
+//      goes round through shared memory.
+//   3. R[J, c] = R_JJ^{-T} G[J, c] beyond the block by forward substitution, a lane per
+//      column with its 32 values in registers (the pivots' reciprocals are formed
+//      once).
+// The chain of pivots bounds small sizes and step 1's operations on one SM large ones.
+// Measured (one warp per column with a lane per row for steps 1 and 3 before): k = 48
+// 47 -> 12 us, 128 90 -> 46 us, 288 772 -> 207 us.
+constexpr int kPotrfNB = 32;
+constexpr int kPotrfThreads = 512;
+constexpr int kPotrfLd = 40;     // 4 rows x 8 columns of a fragment: two wavefronts
+constexpr int kPotrfStage = 512;  // rows of R[0:j0, J] staged at once
+constexpr size_t potrf_smem(int k) {
+  const int rows = k < kPotrfStage ? k : kPotrfStage;
+  return (static_cast<size_t>(rows) * kPotrfLd + 32 * 33 + 64) * sizeof(double);
 }
 
-// Blocked left-looking Cholesky (upper, G = R^T R) in one CTA of 32 warps, with
-// 32-column panels. For panel J (columns j0..j0+jb):
-//   1. G[J, c] -= R[0:j0, J]^T R[0:j0, c] for every c >= j0: one warp per column c,
-//      lane r owns row j0+r; R[0:j0, J] sits in shared memory, R[l, c] is a
-//      broadcast load. Only the upper triangle of the diagonal block is used.
-//   2. warp 0 factors the jb x jb diagonal block in registers/shared memory.
-//   3. R[J, c] = R_JJ^{-T} G[J, c] for c >= j0+jb: forward substitution with
-//      shuffles, one warp per column.
-// Dynamic shared memory: k*32 doubles (panel) + 32*33 doubles (diagonal block).
-constexpr int kPotrfNB = 32;
+__device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(d[0]), "+d"(d[1])
+               : "d"(a), "d"(b));
+}
 
-__global__ void __launch_bounds__(1024)
-potrf_upper_blocked_kernel(double* G, int k, int64_t ldg, int32_t* info, int64_t batch_stride) {
+__global__ void __launch_bounds__(kPotrfThreads)
+potrf_upper_kernel(double* G, int k, int64_t ldg, int32_t* info, int64_t batch_stride) {
   // batched: CTA b factors the matrix batch_stride doubles after the previous one
   G += static_cast<int64_t>(blockIdx.x) * batch_stride;
   if (info) info += blockIdx.x;
   extern __shared__ double psm[];
-  double* panel = psm;                      // [k][32]: panel[l * 32 + r] = R[l, j0 + r]
-  double* diag = psm + static_cast<size_t>(k) * kPotrfNB;  // [32][33]
+  double* diag = psm;                // [32][33]: R_JJ by rows
+  double* rinv = diag + 32 * 33;     // [32]: reciprocals of its diagonal
+  double* panel = rinv + 64;         // [rows][kPotrfLd]: panel[l][r] = R[l, j0 + r]
   __shared__ int failed;
-  const int warp = threadIdx.x / 32;
-  const int lane = threadIdx.x % 32;
-  const int nwarps = blockDim.x / 32;
-  if (threadIdx.x == 0) failed = 0;
-  __syncthreads();
-  auto g = [&](int r, int c) -> double& { return G[static_cast<int64_t>(c) * ldg + r]; };
+  const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  constexpr int kWarps = kPotrfThreads / 32;
+  const int fq = lane & 3, fp = lane >> 2;
+  if (tid == 0) failed = 0;
   for (int j0 = 0; j0 < k; j0 += kPotrfNB) {
     const int jb = min(kPotrfNB, k - j0);
-    // stage R[0:j0, J] (already final) into shared memory
-    for (int idx = threadIdx.x; idx < j0 * kPotrfNB; idx += blockDim.x) {
-      const int l = idx / kPotrfNB;
-      const int r = idx % kPotrfNB;
-      panel[idx] = (r < jb) ? g(l, j0 + r) : 0.0;
-    }
-    __syncthreads();
-    // 1. update the panel row against the finished rows 0..j0-1
-    for (int c = j0 + warp; c < k; c += nwarps) {
-      if (lane < jb && j0 + lane <= c) {
-        double acc = 0.0;
-        for (int l = 0; l < j0; ++l) acc = fma(panel[l * kPotrfNB + lane], g(l, c), acc);
-        g(j0 + lane, c) -= acc;
+    for (int l0 = 0; l0 < j0; l0 += kPotrfStage) {
+      const int rows = min(kPotrfStage, j0 - l0);  // a multiple of 32
+      __syncthreads();
+      for (int idx = tid; idx < rows * kPotrfNB; idx += kPotrfThreads) {
+        const int r = idx / rows, l = idx - r * rows;
+        panel[l * kPotrfLd + r] =
+            r < jb ? G[static_cast<int64_t>(j0 + r) * ldg + l0 + l] : 0.0;
+      }
+      __syncthreads();
+      for (int c = j0 + warp * 8; c < k; c += kWarps * 8) {
+        const double* gc = G + static_cast<int64_t>(min(c + fp, k - 1)) * ldg + l0 + fq;
+        double acc[4][2] = {};
+        double b[8], bn[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) bn[u] = gc[u * 4];
+        for (int l = 0; l < rows; l += 32) {
+#pragma unroll
+          for (int u = 0; u < 8; ++u) b[u] = bn[u];
+          if (l + 32 < rows) {
+#pragma unroll
+            for (int u = 0; u < 8; ++u) bn[u] = gc[l + 32 + u * 4];
+          }
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            const double* pl = panel + (l + u * 4 + fq) * kPotrfLd + fp;
+#pragma unroll
+            for (int m = 0; m < 4; ++m) dmma_8x8x4(acc[m], pl[m * 8], b[u]);
+          }
+        }
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int r = m * 8 + fp, col = c + 2 * fq + e;
+            if (r < jb && col < k && j0 + r <= col)
+              G[static_cast<int64_t>(col) * ldg + j0 + r] -= acc[m][e];
+          }
       }
     }
     __syncthreads();
-    // 2. factor the diagonal block (warp 0, column by column)
     if (warp == 0) {
-      for (int c = 0; c < jb; ++c)
-        if (lane <= c) diag[lane * 33 + c] = g(j0 + lane, j0 + c);
-      __syncwarp();
-      for (int j = 0; j < jb; ++j) {
-        double d = diag[j * 33 + j];
-        const bool bad = !(d > 0.0) || !isfinite(d);
-        if (bad) {
-          if (lane == 0) failed = j0 + j + 1;
-          break;
-        }
-        const double r = sqrt(d);
+      // a lane per column of the diagonal block, padded with the identity
+      double a[32];
+      const double* gc = G + static_cast<int64_t>(j0 + lane) * ldg + j0;
+#pragma unroll
+      for (int r = 0; r < 32; ++r)
+        a[r] = lane < jb && r <= lane ? gc[r] : (r == lane ? 1.0 : 0.0);
+      int bad = 0;
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        const double d = __shfl_sync(0xffffffffu, a[j], j);
+        if (bad == 0 && (!(d > 0.0) || !isfinite(d))) bad = j + 1;
+        const double root = sqrt(d), inv = 1.0 / root;
+        const double v = lane == j ? root : a[j] * inv;
+        a[j] = v;
+        diag[j * 33 + lane] = v;
+        if (lane == 0) rinv[j] = inv;
         __syncwarp();
-        if (lane == j) diag[j * 33 + j] = r;
-        if (lane > j && lane < jb) diag[j * 33 + lane] /= r;
-        __syncwarp();
-        // trailing update of the block's upper triangle: a = lane, columns c >= a
-        if (lane > j && lane < jb) {
-          const double rja = diag[j * 33 + lane];
-          for (int c = lane; c < jb; ++c) diag[lane * 33 + c] -= rja * diag[j * 33 + c];
-        }
-        __syncwarp();
+#pragma unroll
+        for (int r = j + 1; r < 32; ++r) a[r] = fma(-diag[j * 33 + r], v, a[r]);
+        asm volatile("" ::: "memory");
       }
-      __syncwarp();
-      if (!failed) {
-        for (int c = 0; c < jb; ++c)
-          if (lane <= c) g(j0 + lane, j0 + c) = diag[lane * 33 + c];
+      if (bad) {
+        if (lane == 0) failed = j0 + bad;
+      } else if (lane < jb) {
+        double* go = G + static_cast<int64_t>(j0 + lane) * ldg + j0;
+#pragma unroll
+        for (int r = 0; r < 32; ++r)
+          if (r <= lane) go[r] = a[r];
       }
     }
     __syncthreads();
     if (failed) break;
-    // 3. triangular solve for the rest of the panel row: R_JJ^T x = G[J, c]
-    for (int c = j0 + jb + warp; c < k; c += nwarps) {
-      double x = (lane < jb) ? g(j0 + lane, c) : 0.0;
-      for (int i = 0; i < jb; ++i) {
-        const double xi = __shfl_sync(0xffffffffu, x, i) / diag[i * 33 + i];
-        if (lane == i) x = xi;
-        if (lane > i && lane < jb) x -= diag[i * 33 + lane] * xi;
+    for (int c = j0 + jb + tid; c < k; c += kPotrfThreads) {
+      double* gc = G + static_cast<int64_t>(c) * ldg + j0;  // jb == 32 here
+      double x[32];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) x[i] = gc[i];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        x[i] *= rinv[i];
+#pragma unroll
+        for (int l = i + 1; l < 32; ++l) x[l] = fma(-diag[i * 33 + l], x[i], x[l]);
+        asm volatile("" ::: "memory");  // the next row's loads stay behind: registers
       }
-      if (lane < jb) g(j0 + lane, c) = x;
+#pragma unroll
+      for (int i = 0; i < 32; ++i) gc[i] = x[i];
+    }
+  }
+  __syncthreads();
+  // zero the strict lower triangle
+  for (int c = warp; c < k; c += kWarps)
+    for (int r = c + 1 + lane; r < k; r += 32) G[static_cast<int64_t>(c) * ldg + r] = 0.0;
+  if (tid == 0 && info) *info = failed;
+}
+
+// R^{-1} of an upper triangular R: a CTA per block column J of 32 columns, from its
+// diagonal block up: X_IJ = -R_II^{-1} sum_{L=I+1..J} R_IL X_LJ. The products run on the
+// FP64 tensor cores with X in shared memory and R streamed from L2, the solve with R_II by
+// back substitution, a lane per column. The block columns run side by side, so the longest
+// chain is k / 32 blocks (one warp per column with a dot product per row before: k = 48
+// 28 -> 9 us, 288 340 -> 47 us).
+constexpr int kTrinvThreads = 256;
+constexpr int kTrinvLd = 40;
+constexpr int kTrinvMax = 608;  // rows of X that fit shared memory
+constexpr size_t trinv_smem(int k) {
+  return (static_cast<size_t>((k + 31) / 32 * 32) * kTrinvLd + 2 * 32 * 33 + 32) * sizeof(double);
+}
+
+__global__ void __launch_bounds__(kTrinvThreads)
+trinv_upper_block_kernel(const double* __restrict__ R, int64_t ldr, double* __restrict__ Rinv,
+                         int64_t ldi, int k, int64_t batch_stride) {
+  R += static_cast<int64_t>(blockIdx.y) * batch_stride;
+  Rinv += static_cast<int64_t>(blockIdx.y) * batch_stride;
+  extern __shared__ double tsm[];
+  double* S = tsm;            // [32][33]: the block being solved
+  double* D = S + 32 * 33;    // [32][33]: R_II by rows
+  double* inv = D + 32 * 33;  // [32]: reciprocals of R_II's diagonal
+  double* X = inv + 32;       // [l][kTrinvLd]: X[l][c] = R^{-1}[l, J * 32 + c]
+  const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  const int fq = lane & 3, fp = lane >> 2;
+  // the longest block columns first
+  const int J = static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x);
+  const int cb = min(32, k - J * 32);
+  for (int I = J; I >= 0; --I) {
+    // R_II (padded with the identity) and, for the warps' two tiles each, the products
+    for (int idx = tid; idx < 32 * 32; idx += kTrinvThreads) {
+      const int c = idx / 32, r = idx % 32;
+      const int gr = I * 32 + r, gcol = I * 32 + c;
+      D[r * 33 + c] = gr < k && gcol < k && r <= c ? R[static_cast<int64_t>(gcol) * ldr + gr]
+                                                   : (r == c ? 1.0 : 0.0);
+    }
+    // 16 tiles of 8 x 8: warp w takes rows 8 (w % 4), columns 16 (w / 4) and the next 8
+    const int m0 = (warp & 3) * 8, n0 = (warp >> 2) * 16;
+    double acc[2][2] = {};
+    const double* ra = R + I * 32 + m0 + fp;
+    for (int l = (I + 1) * 32; l < (J + 1) * 32; l += 16) {
+      double a[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        a[u] = l + u * 4 + fq < k ? ra[static_cast<int64_t>(l + u * 4 + fq) * ldr] : 0.0;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const double* xb = X + (l + u * 4 + fq) * kTrinvLd + n0 + fp;
+        dmma_8x8x4(acc[0], a[u], xb[0]);
+        dmma_8x8x4(acc[1], a[u], xb[8]);
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < 2; ++t)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int r = m0 + fp, c = n0 + t * 8 + 2 * fq + e;
+        S[r * 33 + c] = I == J ? (r == c ? 1.0 : 0.0) : -acc[t][e];
+      }
+    __syncthreads();
+    if (warp == 0) {
+      double x[32];
+      inv[lane] = 1.0 / D[lane * 33 + lane];
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < 32; ++i) x[i] = S[i * 33 + lane];
+#pragma unroll
+      for (int i = 31; i >= 0; --i) {
+        x[i] *= inv[i];
+#pragma unroll
+        for (int l = 0; l < i; ++l) x[l] = fma(-D[l * 33 + i], x[i], x[l]);
+      }
+#pragma unroll
+      for (int i = 0; i < 32; ++i) X[(I * 32 + i) * kTrinvLd + lane] = x[i];
     }
     __syncthreads();
   }
-  // zero the strict lower triangle
-  for (int64_t idx = threadIdx.x; idx < static_cast<int64_t>(k) * k; idx += blockDim.x) {
-    const int r = static_cast<int>(idx % k);
-    const int c = static_cast<int>(idx / k);
-    if (r > c) g(r, c) = 0.0;
+  for (int c = warp; c < cb; c += kTrinvThreads / 32) {
+    const int col = J * 32 + c;
+    for (int r = lane; r < k; r += 32)
+      Rinv[static_cast<int64_t>(col) * ldi + r] = r <= col ? X[r * kTrinvLd + c] : 0.0;
   }
-  if (threadIdx.x == 0 && info) *info = failed;
 }
 
 // One warp per column c of Rinv: back substitution R x = e_c.
@@ -497,26 +572,45 @@ __global__ void symmetrize_kernel(double* P, int k, int64_t ldp, int64_t batch_s
 
 }  // namespace
 
+namespace {
+
+void launch_potrf(double* G, int k, int64_t ldg, int32_t* info, int64_t stride, int64_t count,
+                  cudaStream_t s) {
+  FE_CHECK_CUDA(cudaFuncSetAttribute(potrf_upper_kernel,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     static_cast<int>(potrf_smem(kPotrfStage))));
+  potrf_upper_kernel<<<static_cast<unsigned>(count), kPotrfThreads, potrf_smem(k), s>>>(
+      G, k, ldg, info, stride);
+  check_launch("potrf_upper_kernel");
+}
+
+void launch_trinv(const double* R, int64_t ldr, double* Rinv, int64_t ldi, int k, int64_t stride,
+                  int64_t count, cudaStream_t s) {
+  if (k <= kTrinvMax) {
+    FE_CHECK_CUDA(cudaFuncSetAttribute(trinv_upper_block_kernel,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       static_cast<int>(trinv_smem(kTrinvMax))));
+    const dim3 grid(static_cast<unsigned>((k + 31) / 32), static_cast<unsigned>(count));
+    trinv_upper_block_kernel<<<grid, kTrinvThreads, trinv_smem(k), s>>>(R, ldr, Rinv, ldi, k,
+                                                                       stride);
+    check_launch("trinv_upper_block_kernel");
+    return;
+  }
+  const int64_t threads = static_cast<int64_t>(k) * 32;
+  const dim3 grid(static_cast<unsigned>((threads + 255) / 256), static_cast<unsigned>(count));
+  trinv_upper_kernel<<<grid, 256, 0, s>>>(R, ldr, Rinv, ldi, k, stride);
+  check_launch("trinv_upper_kernel");
+}
+
+}  // namespace
+
 void potrf_upper(double* G, int64_t k, int64_t ldg, int32_t* info, cudaStream_t s) {
   FE_REQUIRE(k >= 0 && k <= 16384 && ldg >= k, "potrf_upper: invalid shape");
   if (k == 0) {
     if (info) FE_CHECK_CUDA(cudaMemsetAsync(info, 0, sizeof(int32_t), s));
     return;
   }
-  const size_t smem = (static_cast<size_t>(k) * kPotrfNB + 32 * 33) * sizeof(double);
-  if (smem <= 200 * 1024) {
-    static bool attr = false;
-    if (!attr) {
-      FE_CHECK_CUDA(cudaFuncSetAttribute(potrf_upper_blocked_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-      attr = true;
-    }
-    potrf_upper_blocked_kernel<<<1, 1024, smem, s>>>(G, static_cast<int>(k), ldg, info, 0);
-    check_launch("potrf_upper_blocked_kernel");
-    return;
-  }
-  potrf_upper_kernel<<<1, 1024, 0, s>>>(G, static_cast<int>(k), ldg, info);
-  check_launch("potrf_upper_kernel");
+  launch_potrf(G, static_cast<int>(k), ldg, info, 0, 1, s);
 }
 
 void trinv_upper(const double* R, int64_t ldr, double* Rinv, int64_t ldi, int64_t k,
@@ -524,10 +618,7 @@ void trinv_upper(const double* R, int64_t ldr, double* Rinv, int64_t ldi, int64_
   FE_REQUIRE(k >= 0 && ldr >= k && ldi >= k, "trinv_upper: invalid shape");
   if (k == 0) return;
   FE_REQUIRE(R != Rinv, "trinv_upper: in-place inverse is not supported");
-  const int64_t threads = k * 32;
-  trinv_upper_kernel<<<static_cast<unsigned>((threads + 255) / 256), 256, 0, s>>>(
-      R, ldr, Rinv, ldi, static_cast<int>(k), 0);
-  check_launch("trinv_upper_kernel");
+  launch_trinv(R, ldr, Rinv, ldi, static_cast<int>(k), 0, 1, s);
 }
 
 // Batched forms for grouped solves: `count` k x k matrices `stride` doubles apart,
@@ -536,23 +627,14 @@ void potrf_upper_batched(double* G, int64_t k, int64_t ldg, int64_t stride, int6
                          int32_t* info, cudaStream_t s) {
   FE_REQUIRE(k >= 1 && ldg >= k && count >= 1 && count <= 65535 && stride >= ldg * k,
              "potrf_upper_batched: invalid shape");
-  const size_t smem = (static_cast<size_t>(k) * kPotrfNB + 32 * 33) * sizeof(double);
-  FE_REQUIRE(smem <= 200 * 1024, "potrf_upper_batched: k too large for the blocked kernel");
-  FE_CHECK_CUDA(cudaFuncSetAttribute(potrf_upper_blocked_kernel,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-  potrf_upper_blocked_kernel<<<static_cast<unsigned>(count), 1024, smem, s>>>(
-      G, static_cast<int>(k), ldg, info, stride);
-  check_launch("potrf_upper_blocked_kernel");
+  launch_potrf(G, static_cast<int>(k), ldg, info, stride, count, s);
 }
 
 void trinv_upper_batched(const double* R, int64_t ldr, double* Rinv, int64_t ldi, int64_t k,
                          int64_t stride, int64_t count, cudaStream_t s) {
   FE_REQUIRE(k >= 1 && ldr >= k && ldi >= k && count >= 1 && count <= 65535,
              "trinv_upper_batched: invalid shape");
-  const int64_t threads = k * 32;
-  dim3 grid(static_cast<unsigned>((threads + 255) / 256), static_cast<unsigned>(count));
-  trinv_upper_kernel<<<grid, 256, 0, s>>>(R, ldr, Rinv, ldi, static_cast<int>(k), stride);
-  check_launch("trinv_upper_kernel");
+  launch_trinv(R, ldr, Rinv, ldi, static_cast<int>(k), stride, count, s);
 }
 
 size_t chol_inv_small_smem(int64_t k) {

@@ -547,16 +547,13 @@ void rotate_block(SmallState& sm, const T* X, int64_t ldx, const double* C, T* Y
   rotate<T>(X, ldx, C, sm.cap, Y, ldy, n, k, m, alpha, beta, s, upper_tri);
 }
 
-// R^{-1} of chol(G) into Rinv, info as potrf_upper: one fused shared-memory launch for
-// k <= 128; otherwise the factorization in G (which then holds R) and the inverse.
+// R^{-1} of chol(G) into Rinv, info as potrf_upper: the factorization in G (which then holds
+// R) and the inverse, two launches (64 columns 27 us, 128 columns 71 us; the batched fused
+// kernel 58 and 170 us).
 void chol_inverse(double* G, int64_t k, int64_t ldg, double* Rinv, int64_t ldi, int32_t* info,
                   cudaStream_t s) {
-  if (chol_inv_small_fits(k)) {
-    chol_inv_upper_batched(G, k, ldg, 0, Rinv, ldi, 0, 1, info, s);
-  } else {
-    potrf_upper(G, k, ldg, info, s);
-    trinv_upper(G, ldg, Rinv, ldi, k, s);
-  }
+  potrf_upper(G, k, ldg, info, s);
+  trinv_upper(G, ldg, Rinv, ldi, k, s);
 }
 
 // Cholesky QR of src (n x k) into dst: G = src^T src, R = chol(G), dst = src R^{-1}
