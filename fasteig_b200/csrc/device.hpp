@@ -337,7 +337,7 @@ void bks_lanczos_step(const BatchLayout& L, const BatchState& S, const Csr& A, d
                       int64_t ldv, double* f, double* q, double* w, cudaStream_t s);
 void bks_init_norm(const BatchLayout& L, const BatchState& S, const double* f, cudaStream_t s);
 void bks_jacobi(const BatchLayout& L, const double* T, const int32_t* mdim, const int32_t* todo,
-                int max_m, double* W, double* Z, double* Zlast, cudaStream_t s);
+                int max_m, double* W, double* Z, double* Zlast, cudaStream_t s, int same = 0);
 void bks_restart(const BatchLayout& L, const int32_t* mdim, const int32_t* idx,
                  const int32_t* keep, const int32_t* keepY, const double* diag,
                  const double* coup, const double* Z, double* C, double* T, cudaStream_t s);
