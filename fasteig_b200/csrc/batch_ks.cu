@@ -301,14 +301,18 @@ __global__ void bks_end_kernel(BatchLayout L, BatchState S) {
 //
 // A round is bound by shared-memory traffic and by the barriers around it. Each thread takes
 // the 2 x 2 blocks (pair, pair) of A through both sides of the rotation in registers, so A
-// goes through shared memory once a round, not twice, and a round has two barriers; blocks
-// and Q's elements are dealt to 1024 threads once, before the sweeps (8 matrices of 96:
-// 4.01 ms with one side after the other on 256 threads, 1.30 ms so, the same results bit
-// for bit).
+// goes through shared memory once a round, not twice, and a round has two barriers; the
+// next round's rotations (a chain of divisions and roots) are formed beside Q's update;
+// blocks and Q's elements are dealt to 1024 threads once, before the sweeps (a call of 8
+// matrices of 96: 4.76 ms with one side after the other on 256 threads, 1.80 ms so, the
+// same results bit for bit).
 constexpr int kJacThreads = 1024;
 constexpr int kJacMaxHalf = kBatchMaxDim / 2;
 constexpr int kJacBlocks = (kJacMaxHalf * kJacMaxHalf + kJacThreads - 1) / kJacThreads;
-constexpr int kJacQ = (kJacMaxHalf * kBatchMaxDim + kJacThreads - 1) / kJacThreads;
+constexpr int kJacRotThreads = 64;  // form the next round's rotations beside Q's update
+constexpr int kJacQThreads = kJacThreads - kJacRotThreads;
+constexpr int kJacQ = (kJacMaxHalf * kBatchMaxDim + kJacQThreads - 1) / kJacQThreads;
+static_assert(kJacMaxHalf <= kJacRotThreads, "a thread per rotation");
 
 __global__ void __launch_bounds__(kJacThreads)
 bks_jacobi_kernel(BatchLayout L, const double* __restrict__ T, const int32_t* __restrict__ mdim,
@@ -322,8 +326,8 @@ bks_jacobi_kernel(BatchLayout L, const double* __restrict__ T, const int32_t* __
   double* A = sh;
   double* Q = sh + m * ld;
   double2* rot = reinterpret_cast<double2*>(
-      (reinterpret_cast<uintptr_t>(Q + m * ld) + 15) & ~uintptr_t(15));  // (c, s) of a pair
-  int2* pq = reinterpret_cast<int2*>(rot + kJacMaxHalf);                 // its rows
+      (reinterpret_cast<uintptr_t>(Q + m * ld) + 15) & ~uintptr_t(15));  // (c, s) of a pair, two rounds
+  int2* pq = reinterpret_cast<int2*>(rot + 2 * kJacMaxHalf);             // its rows
   __shared__ double red[2][kJacThreads / 32];
   __shared__ int done;
   const int tid = threadIdx.x;
@@ -345,9 +349,36 @@ bks_jacobi_kernel(BatchLayout L, const double* __restrict__ T, const int32_t* __
   }
 #pragma unroll
   for (int u = 0; u < kJacQ; ++u) {
-    const int e = tid + u * kJacThreads;
-    qel[u] = e < half * m ? (e / m) | ((e % m) << 16) : -1;
+    const int e = tid - kJacRotThreads + u * kJacQThreads;
+    qel[u] = tid >= kJacRotThreads && e < half * m ? (e / m) | ((e % m) << 16) : -1;
   }
+  auto rotations = [&](int round) {  // pair tid of the round
+    const int k = tid;
+    int a, b;
+    if (k == 0) {
+      a = round;
+      b = mm - 1;
+    } else {
+      a = round + k;
+      if (a >= mm - 1) a -= mm - 1;
+      b = round - k;
+      if (b < 0) b += mm - 1;
+    }
+    const int lo = min(a, b), hi = max(a, b);
+    double c = 1.0, s = 0.0;
+    if (hi < m) {
+      const double apq = A[lo + hi * ld];
+      if (apq != 0.0) {
+        const double theta = (A[hi + hi * ld] - A[lo + lo * ld]) / (2.0 * apq);
+        const double t = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
+        c = 1.0 / sqrt(t * t + 1.0);
+        s = t * c;
+      }
+    }
+    const int at = (round & 1) * kJacMaxHalf + k;
+    rot[at] = make_double2(c, s);
+    pq[at] = make_int2(lo, hi < m ? hi : lo);
+  };
   for (int sweep = 0; sweep < 40; ++sweep) {
     double off = 0.0, dg = 0.0;
     for (int e = tid; e < m * m; e += kJacThreads) {
@@ -375,39 +406,18 @@ bks_jacobi_kernel(BatchLayout L, const double* __restrict__ T, const int32_t* __
     }
     __syncthreads();
     if (done) break;
+    if (tid < half) rotations(0);
+    __syncthreads();
     for (int round = 0; round < mm - 1; ++round) {
-      if (tid < half) {
-        const int k = tid;
-        int a, b;
-        if (k == 0) {
-          a = round;
-          b = mm - 1;
-        } else {
-          a = (round + k) % (mm - 1);
-          b = (round - k + (mm - 1)) % (mm - 1);
-        }
-        const int lo = min(a, b), hi = max(a, b);
-        double c = 1.0, s = 0.0;
-        if (hi < m) {
-          const double apq = A[lo + hi * ld];
-          if (apq != 0.0) {
-            const double theta = (A[hi + hi * ld] - A[lo + lo * ld]) / (2.0 * apq);
-            const double t = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-            c = 1.0 / sqrt(t * t + 1.0);
-            s = t * c;
-          }
-        }
-        rot[k] = make_double2(c, s);
-        pq[k] = make_int2(lo, hi < m ? hi : lo);
-      }
-      __syncthreads();
+      const double2* rr = rot + (round & 1) * kJacMaxHalf;
+      const int2* rp = pq + (round & 1) * kJacMaxHalf;
       // A <- J^T (A J), block by block
 #pragma unroll
       for (int u = 0; u < kJacBlocks; ++u) {
         if (blk[u] < 0) continue;
         const int k1 = blk[u] & 0xffff, k2 = blk[u] >> 16;
-        const double2 r1 = rot[k1], r2 = rot[k2];
-        const int2 i = pq[k1], j = pq[k2];
+        const double2 r1 = rr[k1], r2 = rr[k2];
+        const int2 i = rp[k1], j = rp[k2];
         const bool id1 = r1.y == 0.0 && r1.x == 1.0, id2 = r2.y == 0.0 && r2.x == 1.0;
         if (id1 && id2) continue;
         double* ca = A + j.x * ld;
@@ -432,14 +442,16 @@ bks_jacobi_kernel(BatchLayout L, const double* __restrict__ T, const int32_t* __
           cb[i.y] = r1.y * tb + r1.x * ub;
         }
       }
-      // Q <- Q J
+      __syncthreads();
+      // Q <- Q J, and the next round's rotations from the new A
+      if (tid < half && round + 1 < mm - 1) rotations(round + 1);
 #pragma unroll
       for (int u = 0; u < kJacQ; ++u) {
         if (qel[u] < 0) continue;
         const int k = qel[u] & 0xffff, i = qel[u] >> 16;
-        const double2 r = rot[k];
+        const double2 r = rr[k];
         if (r.y == 0.0 && r.x == 1.0) continue;
-        const int2 j = pq[k];
+        const int2 j = rp[k];
         const double x = Q[i + j.x * ld], y = Q[i + j.y * ld];
         Q[i + j.x * ld] = r.x * x - r.y * y;
         Q[i + j.y * ld] = r.y * x + r.x * y;
@@ -674,8 +686,8 @@ void bks_init_norm(const BatchLayout& L, const BatchState& S, const double* f, c
 }
 
 size_t bks_jacobi_smem(int m) {
-  return (2 * static_cast<size_t>(m) * (m + 1) + kBatchMaxDim) * sizeof(double) + 16 +
-         kBatchMaxDim * sizeof(int);
+  return (2 * static_cast<size_t>(m) * (m + 1)) * sizeof(double) + 16 +
+         2 * kJacMaxHalf * (sizeof(double2) + sizeof(int2));
 }
 
 void bks_jacobi(const BatchLayout& L, const double* T, const int32_t* mdim, const int32_t* todo,
