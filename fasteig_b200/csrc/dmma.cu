@@ -51,29 +51,31 @@ __device__ __forceinline__ void cp_async_wait() {
 }
 
 // ------------------------------------------------------------------ Gram ----
-// CTA: 64 x 64 output tile (the 64-column tiles of the SIMT plan), 4 warps in
-// 2 x 2, each warp 32 x 32 (4 x 4 m8n8 tiles); 16 rows per stage, 4 stages.
-// Shared rows are 72 doubles: a fragment load (4 rows x 8 consecutive doubles)
-// then falls into two 128-byte wavefronts, the minimum for 256 bytes.
-constexpr int kGT = 64;
+// CTA: T x T output tile, 4 warps in 2 x 2, each warp T/2 x T/2 in m8n8 tiles; 16 rows
+// per stage, 4 stages. Shared rows are T + 8 doubles: a fragment load (4 rows x 8
+// consecutive doubles) then falls into two 128-byte wavefronts, the minimum for 256 bytes.
+// What bounds it is the FP64 tensor pipe, so the tile (gram_dmma_tile) is the one that
+// computes the least beyond the wanted entries.
 constexpr int kGR = 16;
 constexpr int kGStages = 4;
-constexpr int kGLd = 72;
 constexpr int kGThreads = 128;
-constexpr size_t kGSmem = size_t(kGStages) * 2 * kGR * kGLd * sizeof(double);
+constexpr size_t gram_smem(int tile) {
+  return size_t(kGStages) * 2 * kGR * (tile + 8) * sizeof(double);
+}
 
-template <int VEC>
+template <int VEC, int kGT>
 __global__ void __launch_bounds__(kGThreads)
 gram_dmma_kernel(const double* __restrict__ X, int64_t ldx, const double* __restrict__ Y,
                  int64_t ldy, int64_t n, int k, int m, int64_t rows_per_chunk, int symmetric,
                  double* __restrict__ partial, const int64_t* __restrict__ chunk_rows) {
+  constexpr int kGLd = kGT + 8, W = kGT / 2, F = W / 8;
   if (symmetric && blockIdx.x > blockIdx.y) return;  // lower tiles mirror the upper ones
   extern __shared__ double smem[];
   const int tid = threadIdx.x;
   const int lane = tid & 31;
   const int warp = tid >> 5;
-  const int wi = (warp & 1) * 32;
-  const int wj = (warp >> 1) * 32;
+  const int wi = (warp & 1) * W;
+  const int wj = (warp >> 1) * W;
   const int i0 = blockIdx.x * kGT;
   const int j0 = blockIdx.y * kGT;
   // Equal chunks of rows_per_chunk rows, or (grouped Grams) the row range
@@ -106,11 +108,11 @@ gram_dmma_kernel(const double* __restrict__ X, int64_t ldx, const double* __rest
     }
   };
 
-  double acc[4][4][2];
+  double acc[F][F][2];
 #pragma unroll
-  for (int a = 0; a < 4; ++a)
+  for (int a = 0; a < F; ++a)
 #pragma unroll
-    for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+    for (int b = 0; b < F; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
 
 #pragma unroll
   for (int t = 0; t < kGStages - 1; ++t) {
@@ -128,15 +130,15 @@ gram_dmma_kernel(const double* __restrict__ X, int64_t ldx, const double* __rest
     const double* yd = ys(t % kGStages);
 #pragma unroll
     for (int s4 = 0; s4 < kGR / 4; ++s4) {
-      double av[4], bv[4];
+      double av[F], bv[F];
 #pragma unroll
-      for (int a = 0; a < 4; ++a) av[a] = xd[(s4 * 4 + fr) * kGLd + wi + a * 8 + fc];
+      for (int a = 0; a < F; ++a) av[a] = xd[(s4 * 4 + fr) * kGLd + wi + a * 8 + fc];
 #pragma unroll
-      for (int b = 0; b < 4; ++b) bv[b] = yd[(s4 * 4 + fr) * kGLd + wj + b * 8 + fc];
+      for (int b = 0; b < F; ++b) bv[b] = yd[(s4 * 4 + fr) * kGLd + wj + b * 8 + fc];
 #pragma unroll
-      for (int a = 0; a < 4; ++a)
+      for (int a = 0; a < F; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) dmma(acc[a][b], av[a], bv[b]);
+        for (int b = 0; b < F; ++b) dmma(acc[a][b], av[a], bv[b]);
     }
   }
   cp_async_wait<0>();
@@ -144,10 +146,10 @@ gram_dmma_kernel(const double* __restrict__ X, int64_t ldx, const double* __rest
   // Partial layout [chunk][j][i] (column-major k x m per chunk).
   double* out = partial + static_cast<int64_t>(blockIdx.z) * k * m;
 #pragma unroll
-  for (int a = 0; a < 4; ++a) {
+  for (int a = 0; a < F; ++a) {
     const int i = i0 + wi + a * 8 + fc;
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
+    for (int b = 0; b < F; ++b) {
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         const int j = j0 + wj + b * 8 + 2 * fr + c;
@@ -158,21 +160,21 @@ gram_dmma_kernel(const double* __restrict__ X, int64_t ldx, const double* __rest
 }
 
 // -------------------------------------------------------------- Rotation ----
-// CTA: 128 rows x 64 output columns, 8 warps in 4 x 2, each warp 32 x 32; the
-// inner dimension advances 16 per stage through a 3-stage ring. X rows are
-// staged 20 doubles apart (fragment: 8 rows x 4 doubles -> two wavefronts),
-// C rows 72 apart (4 rows x 8 doubles).
+// CTA: 128 rows x TC output columns, 8 warps in 4 x 2, each warp 32 x TC/2; the inner
+// dimension advances 16 per stage through a 3-stage ring. X rows are staged 20 doubles
+// apart (fragment: 8 rows x 4 doubles -> two wavefronts), C rows TC + 8 apart (4 rows x 8
+// doubles).
 constexpr int kRRows = kRotateRowTile;
-constexpr int kRCols = 64;
 constexpr int kRK = 16;
 constexpr int kRStages = 3;
 constexpr int kRXLd = 20;
-constexpr int kRCLd = 72;
 constexpr int kRThreads = 256;
-constexpr size_t kRStage = size_t(kRRows) * kRXLd + size_t(kRK) * kRCLd;
-constexpr size_t kRSmem = kRStages * kRStage * sizeof(double);
+constexpr size_t rotate_stage(int cols) {
+  return size_t(kRRows) * kRXLd + size_t(kRK) * (cols + 8);
+}
+constexpr size_t rotate_smem(int cols) { return kRStages * rotate_stage(cols) * sizeof(double); }
 
-template <int VEC>
+template <int VEC, int kRCols, bool PAIRS>
 __global__ void __launch_bounds__(kRThreads)
 rotate_dmma_kernel(const double* __restrict__ X, int64_t ldx, const double* __restrict__ C,
                    int64_t ldc, double* __restrict__ Y, int64_t ldy, int64_t n, int k, int m,
@@ -181,12 +183,14 @@ rotate_dmma_kernel(const double* __restrict__ X, int64_t ldx, const double* __re
   // Grouped rotation: row tile t of a concatenated block belongs to problem
   // tile_member[t], whose coefficient matrix starts c_stride doubles further per problem.
   if (tile_member) C += static_cast<int64_t>(tile_member[blockIdx.y]) * c_stride;
+  constexpr int kRCLd = kRCols + 8, W = kRCols / 2, F = W / 8;
+  constexpr size_t kRStage = rotate_stage(kRCols);
   extern __shared__ double smem[];
   const int tid = threadIdx.x;
   const int lane = tid & 31;
   const int warp = tid >> 5;
   const int wr = (warp & 3) * 32;
-  const int wc = (warp >> 2) * 32;
+  const int wc = (warp >> 2) * W;
   const int j0 = blockIdx.x * kRCols;
   const int64_t r0 = static_cast<int64_t>(blockIdx.y) * kRRows;
   // Upper-triangular C (CholQR's R^-1): rows k >= j0 + kRCols are zero for this
@@ -224,11 +228,11 @@ rotate_dmma_kernel(const double* __restrict__ X, int64_t ldx, const double* __re
     }
   };
 
-  double acc[4][4][2];
+  double acc[4][F][2];
 #pragma unroll
   for (int a = 0; a < 4; ++a)
 #pragma unroll
-    for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+    for (int b = 0; b < F; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
 
 #pragma unroll
   for (int t = 0; t < kRStages - 1; ++t) {
@@ -246,15 +250,15 @@ rotate_dmma_kernel(const double* __restrict__ X, int64_t ldx, const double* __re
     const double* cd = cs(t % kRStages);
 #pragma unroll
     for (int s4 = 0; s4 < kRK / 4; ++s4) {
-      double av[4], bv[4];
+      double av[4], bv[F];
 #pragma unroll
       for (int a = 0; a < 4; ++a) av[a] = xd[(wr + a * 8 + fp) * kRXLd + s4 * 4 + fq];
 #pragma unroll
-      for (int b = 0; b < 4; ++b) bv[b] = cd[(s4 * 4 + fq) * kRCLd + wc + b * 8 + fp];
+      for (int b = 0; b < F; ++b) bv[b] = cd[(s4 * 4 + fq) * kRCLd + wc + b * 8 + fp];
 #pragma unroll
       for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) dmma(acc[a][b], av[a], bv[b]);
+        for (int b = 0; b < F; ++b) dmma(acc[a][b], av[a], bv[b]);
     }
   }
   cp_async_wait<0>();
@@ -264,16 +268,27 @@ rotate_dmma_kernel(const double* __restrict__ X, int64_t ldx, const double* __re
     const int64_t r = r0 + wr + a * 8 + fp;
     if (r >= n) continue;
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        const int j = j0 + wc + b * 8 + 2 * fq + c;
+    for (int b = 0; b < F; ++b) {
+      const int j = j0 + wc + b * 8 + 2 * fq;
+      double* y = Y + r * ldy + j;
+      if (PAIRS) {  // aligned output, even column counts: both columns in one store
         if (j < m) {
-          double* y = Y + r * ldy + j;
-          double v = alpha * acc[a][b][c];
-          if (use_beta) v = fma(beta, *y, v);
-          *y = v;
+          double2 v = make_double2(alpha * acc[a][b][0], alpha * acc[a][b][1]);
+          if (use_beta) {
+            const double2 o = *reinterpret_cast<const double2*>(y);
+            v.x = fma(beta, o.x, v.x);
+            v.y = fma(beta, o.y, v.y);
+          }
+          *reinterpret_cast<double2*>(y) = v;
         }
+      } else {
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+          if (j + c < m) {
+            double v = alpha * acc[a][b][c];
+            if (use_beta) v = fma(beta, y[c], v);
+            y[c] = v;
+          }
       }
     }
   }
@@ -281,36 +296,71 @@ rotate_dmma_kernel(const double* __restrict__ X, int64_t ldx, const double* __re
 
 }  // namespace
 
-// Gram partials on the 64 x 64 tile grid of (tiles_k, tiles_m, chunks). With
-// `symmetric` (X and Y the same view) only tiles on and above the diagonal are
-// written; the reduction mirrors the rest.
-void gram_partial_dmma(const double* X, int64_t ldx, const double* Y, int64_t ldy, int64_t n,
-                       int k, int m, int tiles_k, int tiles_m, int chunks, int64_t rows_per_chunk,
-                       bool symmetric, double* partial, cudaStream_t s) {
-  const bool vec2 = aligned16(X) && aligned16(Y) && ldx % 2 == 0 && ldy % 2 == 0 && k % 2 == 0 &&
-                    m % 2 == 0;
-  dim3 grid(tiles_k, tiles_m, chunks);
-  // The attribute is per function and device; setting it is a cheap host call.
-  auto kern = vec2 ? gram_dmma_kernel<2> : gram_dmma_kernel<1>;
-  FE_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kGSmem));
-  kern<<<grid, kGThreads, kGSmem, s>>>(X, ldx, Y, ldy, n, k, m, rows_per_chunk, symmetric ? 1 : 0,
-                                       partial, nullptr);
-  check_launch("gram_dmma_kernel");
+// Tile of the FP64 Gram: the one whose tiles cost least, their area weighed by the rate the
+// kernel reaches with it where it fits (27.9, 30.9 and 31.6 TFLOP/s for 32, 48 and 64 at
+// 512,000 x 288 or 320; 96 x 96 tiles, 29.2, never won). 512,000 rows: 288 columns 2.05 ms
+// in tiles of 64, 1.65 in tiles of 48; 160 columns 866 -> 620 us (32); 96 439 -> 273 us.
+int gram_dmma_tile(int64_t k, int64_t m, bool symmetric) {
+  constexpr int kTiles[] = {32, 48, 64};
+  constexpr double kRate[] = {27.9, 30.9, 31.6};
+  int best = 64;
+  double least = 0.0;
+  for (int t = 0; t < 3; ++t) {
+    const double tk = static_cast<double>((k + kTiles[t] - 1) / kTiles[t]);
+    const double tm = static_cast<double>((m + kTiles[t] - 1) / kTiles[t]);
+    const double tiles = symmetric ? tk * (tk + 1) / 2 : tk * tm;
+    const double cost = tiles * kTiles[t] * kTiles[t] / kRate[t];
+    if (t == 0 || cost < least) {
+      least = cost;
+      best = kTiles[t];
+    }
+  }
+  return best;
 }
 
-// Grouped Gram partials: chunk z covers rows [chunk_rows[2z], chunk_rows[2z+1]) of
-// the concatenated blocks (each chunk inside one problem's rows).
-void gram_partial_dmma_ranges(const double* X, int64_t ldx, const double* Y, int64_t ldy, int k,
-                              int m, int chunks, const int64_t* chunk_rows, bool symmetric,
-                              double* partial, cudaStream_t s) {
+namespace {
+
+// Column tile of the rotation: the one that multiplies least past the output's columns and,
+// for an upper triangular C, below its diagonal; all reach 28 to 30 TFLOP/s, so ties go to
+// the first here. 512,000 rows, k = m: 288 columns 3.30 ms in tiles of 64, 2.87 in tiles of
+// 96; 160 columns 1.14 -> 0.94 ms (32).
+int rotate_tile(int64_t k, int64_t m, bool upper_tri) {
+  constexpr int kTiles[] = {96, 32, 80, 48};
+  int best = 32;
+  int64_t least = -1;
+  for (int t : kTiles) {
+    int64_t cost = 0;
+    for (int64_t j = 0; j < m; j += t) cost += t * (upper_tri ? std::min<int64_t>(k, j + t) : k);
+    if (least < 0 || cost < least) {
+      least = cost;
+      best = t;
+    }
+  }
+  return best;
+}
+
+}  // namespace
+
+// Gram partials on the tile x tile grid of (k, m) and `chunks` row chunks. With `symmetric`
+// (X and Y the same view) only tiles on and above the diagonal are written; the reduction
+// mirrors the rest.
+void gram_partial_dmma(const double* X, int64_t ldx, const double* Y, int64_t ldy, int64_t n,
+                       int k, int m, int tile, int chunks, int64_t rows_per_chunk,
+                       const int64_t* chunk_rows, bool symmetric, double* partial,
+                       cudaStream_t s) {
   const bool vec2 = aligned16(X) && aligned16(Y) && ldx % 2 == 0 && ldy % 2 == 0 && k % 2 == 0 &&
                     m % 2 == 0;
-  FE_REQUIRE(chunks >= 1 && chunks <= 65535, "grouped Gram: chunk count out of range");
-  dim3 grid((k + kGT - 1) / kGT, (m + kGT - 1) / kGT, chunks);
-  auto kern = vec2 ? gram_dmma_kernel<2> : gram_dmma_kernel<1>;
-  FE_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kGSmem));
-  kern<<<grid, kGThreads, kGSmem, s>>>(X, ldx, Y, ldy, 0, k, m, 0, symmetric ? 1 : 0, partial,
-                                       chunk_rows);
+  FE_REQUIRE(chunks >= 1 && chunks <= 65535, "Gram: chunk count out of range");
+  const dim3 grid((k + tile - 1) / tile, (m + tile - 1) / tile, chunks);
+  auto run = [&](auto kern, int t) {
+    FE_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       static_cast<int>(gram_smem(t))));
+    kern<<<grid, kGThreads, gram_smem(t), s>>>(X, ldx, Y, ldy, n, k, m, rows_per_chunk,
+                                               symmetric ? 1 : 0, partial, chunk_rows);
+  };
+  if (tile == 32) vec2 ? run(gram_dmma_kernel<2, 32>, 32) : run(gram_dmma_kernel<1, 32>, 32);
+  else if (tile == 48) vec2 ? run(gram_dmma_kernel<2, 48>, 48) : run(gram_dmma_kernel<1, 48>, 48);
+  else vec2 ? run(gram_dmma_kernel<2, 64>, 64) : run(gram_dmma_kernel<1, 64>, 64);
   check_launch("gram_dmma_kernel");
 }
 
@@ -318,20 +368,33 @@ void rotate_dmma(const double* X, int64_t ldx, const double* C, int64_t ldc, dou
                  int64_t ldy, int64_t n, int64_t k, int64_t m, double alpha, double beta,
                  cudaStream_t s, bool upper_tri, const int32_t* tile_member, int64_t c_stride) {
   const bool vec2 = aligned16(X) && ldx % 2 == 0 && k % 2 == 0;
+  const bool pairs = vec2 && aligned16(Y) && ldy % 2 == 0 && m % 2 == 0;
+  const int cols = rotate_tile(k, m, upper_tri);
   const int64_t row_tiles = (n + kRRows - 1) / kRRows;
-  const int64_t col_tiles = (m + kRCols - 1) / kRCols;
+  const int64_t col_tiles = (m + cols - 1) / cols;
   FE_REQUIRE(col_tiles <= 65535, "rotate: too many columns");
-  auto kern = vec2 ? rotate_dmma_kernel<2> : rotate_dmma_kernel<1>;
-  FE_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kRSmem));
   // Column tiles run fastest so the CTAs sharing an X row tile are adjacent (L2 reuse).
   for (int64_t base = 0; base < row_tiles; base += 65535) {
     const int64_t tiles = std::min<int64_t>(65535, row_tiles - base);
     dim3 grid(static_cast<unsigned>(col_tiles), static_cast<unsigned>(tiles));
     const int64_t r_off = base * kRRows;
-    kern<<<grid, kRThreads, kRSmem, s>>>(X + r_off * ldx, ldx, C, ldc, Y + r_off * ldy, ldy,
-                                         n - r_off, static_cast<int>(k), static_cast<int>(m),
-                                         alpha, beta, beta != 0.0 ? 1 : 0, upper_tri ? 1 : 0,
-                                         tile_member ? tile_member + base : nullptr, c_stride);
+    auto run = [&](auto kern, int t) {
+      FE_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(rotate_smem(t))));
+      kern<<<grid, kRThreads, rotate_smem(t), s>>>(
+          X + r_off * ldx, ldx, C, ldc, Y + r_off * ldy, ldy, n - r_off, static_cast<int>(k),
+          static_cast<int>(m), alpha, beta, beta != 0.0 ? 1 : 0, upper_tri ? 1 : 0,
+          tile_member ? tile_member + base : nullptr, c_stride);
+    };
+#define FE_ROT(TC_)                                                                        \
+  (pairs ? run(rotate_dmma_kernel<2, TC_, true>, TC_)                                      \
+         : vec2 ? run(rotate_dmma_kernel<2, TC_, false>, TC_)                              \
+                : run(rotate_dmma_kernel<1, TC_, false>, TC_))
+    if (cols == 32) FE_ROT(32);
+    else if (cols == 48) FE_ROT(48);
+    else if (cols == 80) FE_ROT(80);
+    else FE_ROT(96);
+#undef FE_ROT
     check_launch("rotate_dmma_kernel");
   }
 }

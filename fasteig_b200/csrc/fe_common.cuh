@@ -146,16 +146,17 @@ void launch_wait_probe(int* status, long long limit_cycles, int code, cudaStream
 int* thread_status_word();
 
 // FP64 tensor-core kernels (dmma.cu).
+int gram_dmma_tile(int64_t k, int64_t m, bool symmetric);
 void gram_partial_dmma(const double* X, int64_t ldx, const double* Y, int64_t ldy, int64_t n,
-                       int k, int m, int tiles_k, int tiles_m, int chunks, int64_t rows_per_chunk,
-                       bool symmetric, double* partial, cudaStream_t s);
+                       int k, int m, int tile, int chunks, int64_t rows_per_chunk,
+                       const int64_t* chunk_rows, bool symmetric, double* partial,
+                       cudaStream_t s);
 void rotate_dmma(const double* X, int64_t ldx, const double* C, int64_t ldc, double* Y,
                  int64_t ldy, int64_t n, int64_t k, int64_t m, double alpha, double beta,
                  cudaStream_t s, bool upper_tri = false, const int32_t* tile_member = nullptr,
                  int64_t c_stride = 0);
-void gram_partial_dmma_ranges(const double* X, int64_t ldx, const double* Y, int64_t ldy, int k,
-                              int m, int chunks, const int64_t* chunk_rows, bool symmetric,
-                              double* partial, cudaStream_t s);
+// Output tile of the grouped Grams (the rule of their reduction).
+constexpr int kGroupGramTile = 64;
 // Row tile of the FP64 rotation kernel (grouped rotations pad every problem's rows
 // to a multiple of it).
 constexpr int kRotateRowTile = 128;

@@ -87,7 +87,7 @@ __global__ void gram_reduce_members_kernel(const double* __restrict__ partial, i
   if (idx >= total) return;
   const int i = static_cast<int>(idx % k);
   const int j = static_cast<int>(idx / k);
-  const int64_t src = (symmetric && i / 64 > j / 64) ? static_cast<int64_t>(i) * k + j : idx;
+  const int64_t src = (symmetric && i / kGroupGramTile > j / kGroupGramTile) ? static_cast<int64_t>(i) * k + j : idx;
   const int c0 = member_chunks[2 * p];
   const int nc = member_chunks[2 * p + 1];
   double s = 0.0;

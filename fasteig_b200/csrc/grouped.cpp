@@ -435,9 +435,9 @@ void ChebGroup::launch_cycle() {
     const int s1 = res == 0 ? 1 : (res == 1 ? 2 : 1);
     const int s2 = res == 0 ? 2 : res;
     auto cholqr = [&](int src, int dst, int32_t* inf) {
-      gram_partial_dmma_ranges(B[src], b, B[src], b, static_cast<int>(b), static_cast<int>(b),
-                               static_cast<int>(I.chunks), I.chunk_rows.as<int64_t>(), true,
-                               I.gpart.as<double>(), s);
+      gram_partial_dmma(B[src], b, B[src], b, 0, static_cast<int>(b), static_cast<int>(b),
+                        kGroupGramTile, static_cast<int>(I.chunks), 0,
+                        I.chunk_rows.as<int64_t>(), true, I.gpart.as<double>(), s);
       group_gram_reduce(I.gpart.as<double>(), static_cast<int>(b), static_cast<int>(b), G,
                         I.member_chunks.as<int32_t>(), true, I.Gm.as<double>(), bb, s);
       potrf_upper_batched(I.Gm.as<double>(), b, b, bb, G, inf, s);
@@ -450,9 +450,9 @@ void ChebGroup::launch_cycle() {
     const int basis = s2;
     // 4. Rayleigh-Ritz
     csr_spmm<double>(I.op_plain, B[basis], b, B[3], b, nullptr, 0, b, 1.0, 0.0, 0.0, s);
-    gram_partial_dmma_ranges(B[basis], b, B[3], b, static_cast<int>(b), static_cast<int>(b),
-                             static_cast<int>(I.chunks), I.chunk_rows.as<int64_t>(), false,
-                             I.gpart.as<double>(), s);
+    gram_partial_dmma(B[basis], b, B[3], b, 0, static_cast<int>(b), static_cast<int>(b),
+                      kGroupGramTile, static_cast<int>(I.chunks), 0,
+                      I.chunk_rows.as<int64_t>(), false, I.gpart.as<double>(), s);
     group_gram_reduce(I.gpart.as<double>(), static_cast<int>(b), static_cast<int>(b), G,
                       I.member_chunks.as<int32_t>(), false, I.Gm.as<double>(), bb, s);
     symmetrize_batched(I.Gm.as<double>(), b, b, bb, G, s);
