@@ -1,20 +1,19 @@
 // Block SpMM and Chebyshev step with several rows to a warp, over bricks of the grid that
 // the operator's diagonals show (sm_100a).
 //
-// A group of G lanes owns a row and reads 16 bytes a lane, so a warp works on 32 / G rows
-// of one column panel (256 or 128 bytes of every row). What bounds it, after DRAM, is the
-// instructions and the load-store wavefronts of an SM rather than the bytes: one warp per
-// row with 8-byte lanes spends them on a row of few columns as on a wide one (96^3 grid,
-// 7 points, FP32 step of 64 columns: 380 us so, 161 us here, 113 us of DRAM traffic at the
-// copy rate). Hence 16-byte lanes, byte pitches in 32 bits (one wide multiply-add per
-// address), all neighbours of a row in flight, and no predicates where the rows of the
-// warp have as many entries.
+// A group of G lanes owns a row and reads up to three 16-byte vectors a lane, so a warp works
+// on 32 / G rows of one column panel. What bounds it, after DRAM, is the instructions and the
+// load-store wavefronts of an SM rather than the bytes: one warp per row with 8-byte lanes
+// spends them on a row of few columns as on a wide one (96^3 grid, 7 points, FP32 step of 64
+// columns: 380 us so, 146 us here, 113 us of DRAM traffic at the copy rate). Hence 16-byte
+// lanes, byte pitches in 32 bits (one wide multiply-add per address), few lanes to a row, and
+// no predicates where the rows of the warp have as many entries.
 //
 // Rows are dealt out in bricks: a CTA's groups take bx x by rows of neighbouring lines and
 // sweep down bz planes, so that the neighbours along a line, across lines and from plane to
 // plane are read while L1 still holds them: 57 % of the loads hit L1 against 24 % for
 // consecutive rows (128^3, FP32 step of 320 columns: 1.91 ms with one warp per row, 2.35 ms
-// with consecutive rows here, 1.70 ms in bricks, 1.27 ms of DRAM traffic). The brick is
+// with consecutive rows here, 1.67 ms in bricks, 1.27 ms of DRAM traffic). The brick is
 // only an order: any strides s1 (line) and s2 (plane, a multiple of s1) number every row
 // once.
 //
@@ -27,6 +26,7 @@
 #include "fe_common.cuh"
 
 #include <algorithm>
+#include <cmath>
 #include <vector>
 
 namespace fe {
@@ -201,9 +201,9 @@ spmm_rows_kernel(const __grid_constant__ RowsParams<T> P) {
         ne2 = __ldg(P.rowptr + nrow2 + 1);
       }
     };
-    auto fetch = [&](int cj, int q) -> V {
+    auto fetch = [&](int cj, int q, bool careful) -> V {
       const T* p = reinterpret_cast<const T*>(at(xp[q], cj, P.ldx));
-      if constexpr (TAIL) {
+      if (TAIL && careful) {
         if (cj == last_x) {
           V r;
 #pragma unroll
@@ -214,7 +214,12 @@ spmm_rows_kernel(const __grid_constant__ RowsParams<T> P) {
       return load_ro<T, VEC>(p);
     };
     const int cnt0 = __shfl_sync(kFull, cnt, 0);
-    if (__all_sync(kFull, cnt == cnt0)) {
+    bool plain = cnt == cnt0;
+    if constexpr (TAIL) {  // rows that touch X's last row take the careful path
+#pragma unroll
+      for (int m = 0; m < M; ++m) plain = plain && c[m] != P.last_x;
+    }
+    if (__all_sync(kFull, plain)) {
       // every row of the warp has as many entries: no lane is held back
 #pragma unroll
       for (int m = 0; m < M; ++m) {
@@ -227,7 +232,7 @@ spmm_rows_kernel(const __grid_constant__ RowsParams<T> P) {
             for (int j = 0; j < KC; ++j) {
               const int cj = __shfl_sync(kFull, c[m], j0 + j, G);
 #pragma unroll
-              for (int q = 0; q < CPL; ++q) xv[j][q] = fetch(cj, q);
+              for (int q = 0; q < CPL; ++q) xv[j][q] = fetch(cj, q, false);
             }
             if (base == 0) prefetch();
 #pragma unroll
@@ -247,7 +252,7 @@ spmm_rows_kernel(const __grid_constant__ RowsParams<T> P) {
                 const T wj = __shfl_sync(kFull, w[m], j0 + j, G);
 #pragma unroll
                 for (int q = 0; q < CPL; ++q) {
-                  const V xv = fetch(cj, q);
+                  const V xv = fetch(cj, q, false);
 #pragma unroll
                   for (int f = 0; f < VEC; ++f) acc[q].v[f] = fma(wj, xv.v[f], acc[q].v[f]);
                 }
@@ -271,7 +276,7 @@ spmm_rows_kernel(const __grid_constant__ RowsParams<T> P) {
           if (m * G + j < cnt) {
 #pragma unroll
             for (int q = 0; q < CPL; ++q) {
-              const V xv = fetch(cj, q);
+              const V xv = fetch(cj, q, true);
 #pragma unroll
               for (int f = 0; f < VEC; ++f) acc[q].v[f] = fma(wj, xv.v[f], acc[q].v[f]);
             }
@@ -284,7 +289,7 @@ spmm_rows_kernel(const __grid_constant__ RowsParams<T> P) {
       if (row >= 0 && !(found & mine)) {
 #pragma unroll
         for (int q = 0; q < CPL; ++q) {
-          const V xv = fetch(row, q);
+          const V xv = fetch(row, q, true);
 #pragma unroll
           for (int f = 0; f < VEC; ++f) acc[q].v[f] = fma(P.gamma, xv.v[f], acc[q].v[f]);
         }
@@ -298,7 +303,7 @@ spmm_rows_kernel(const __grid_constant__ RowsParams<T> P) {
 #pragma unroll
           for (int f = 0; f < VEC; ++f) out.v[f] = P.alpha * out.v[f];
           if (P.use_gamma) {  // the row of X is in L1
-            const V xv = fetch(row, q);
+            const V xv = fetch(row, q, true);
 #pragma unroll
             for (int f = 0; f < VEC; ++f) out.v[f] = fma(P.gamma, xv.v[f], out.v[f]);
           }
@@ -362,10 +367,12 @@ void launch(RowsParams<T> P, int64_t rows, bool tail, cudaStream_t s) {
   P.ny = (P.lines + by - 1) / by;
   const int64_t planes = (rows + P.s2 - 1) / P.s2;
   const int64_t columns = static_cast<int64_t>(P.nx) * P.ny * P.panels;
-  // Deep bricks re-read fewer planes, as long as every SM still gets about three rounds of
-  // its four CTAs.
-  P.bz = 16;
-  while (P.bz > 1 && columns * ((planes + P.bz - 1) / P.bz) < int64_t(12) * num_sms()) P.bz /= 2;
+  // A CTA's first rows wait for a chain of loads that the later ones hide, and deep bricks
+  // re-read fewer planes; but the deeper they are, the longer the last CTAs run alone. With W
+  // rows to each of the four CTAs of every SM, W / d starts and a tail of d are least at
+  // d = sqrt(W) (13 points, 34 FP64 columns, 63^3: 112 us so, 148 us in bricks of 16).
+  const double share = static_cast<double>(columns * planes) / (4.0 * num_sms());
+  P.bz = std::max(1, std::min(16, static_cast<int>(std::sqrt(share) + 0.5)));
   const int64_t grid = columns * ((planes + P.bz - 1) / P.bz);
   FE_REQUIRE(grid <= 0x7fffffffLL, "csr_spmm: too many rows for one launch");
   if (VEC > 1 && tail)
@@ -482,6 +489,26 @@ bool csr_spmm_rows(const Csr& A, const T* X, int64_t ldx, T* Y, int64_t ldy, con
   // as the row kernel of spmm.cu would take it: short rows, 32 or more 8-byte vectors
   const bool fold = k <= 7 && vec * sizeof(T) >= 8 && bytes % 8 == 0 && bytes >= 256;
   const bool tail = ncols % vec != 0;
+  // Where the kernels of spmm.cu are the better ones (us, there and here):
+  // - few rows (94 FP32 columns, 25^3: 13.2, 16.1), small blocks of whole vectors, which
+  //   stay in L2 (16 FP64 columns, 43^3: 12.4, 15.8), larger ones of wide rows (158 FP64
+  //   columns, 29^3: 25, 29; but 100 FP32 columns, 43^3, 32 MB: 40, 31) and of rows of up to
+  //   8 vectors (28 FP32 columns, 57^3: 21, 25; 32, 96^3: 104, 100);
+  // - 17 or more entries a row: rows of more than 48 vectors, whose lanes are full there (124
+  //   FP64 columns, 51^3: 192, 207), blocks of up to 16 whole vectors, whose lanes there are
+  //   fewer (16 FP64 columns, 76^3: 126, 193), and element-wide lanes (49 FP64 columns, 31^3:
+  //   31, 45);
+  // - element-wide lanes: FP32 (113 columns, 57^3: 95, 136); FP64 where the row kernel's lanes
+  //   are full (149 columns, 71^3: 334, 356, but 70 columns, 55^3: 140, 88) and, with longer
+  //   rows, up to 224 columns (193, 42^3: 129, 142, but 275, 38^3: 244, 153).
+  const int64_t block = A.rows * bytes;
+  if (A.rows < 32768) return false;
+  if (!tail && (block < (int64_t(16) << 20) || (bytes >= 1024 && block < (int64_t(32) << 20)) ||
+                (bytes <= 128 && block < (int64_t(64) << 20))))
+    return false;
+  if (k > 16 && (bytes > 768 || vec != V16 || bytes <= (tail ? 128 : 256))) return false;
+  if (vec == 1 && (sizeof(T) == 4 || (k <= 7 ? ncols < 32 || ncols > 96 : ncols <= 224)))
+    return false;
   const int nvec = static_cast<int>((ncols + vec - 1) / vec);
   auto panels = [&](int cap) {
     P.panels = (nvec + cap - 1) / cap;
@@ -499,36 +526,63 @@ bool csr_spmm_rows(const Csr& A, const T* X, int64_t ldx, T* Y, int64_t ldy, con
     FE_ROWS_F(V_, G_, C_, M_, K_, false, CORR_);                \
   } while (0)
   if (vec == V16) {
-    // 128-byte panels where 256-byte ones would leave more than a tenth more lanes idle
-    // (160 FP32 columns: 5 full panels of 128 bytes, 422 us, or 3 of 256, 433 us; 96^3).
-    const int lanes16 = (nvec + 15) / 16 * 16, lanes8 = (nvec + 7) / 8 * 8;
-    const bool narrow = k <= 16 && lanes8 * 10 < lanes16 * 9;
+    // One panel of the fewest lanes and vectors that hold the row, two neighbours in flight:
+    // a row's share of the instructions falls with the vectors of a lane (96^3, 7 points,
+    // FP32, us: 64 columns 146 with (8 lanes, 2 vectors) against 161 with (16, 1), 80 columns
+    // 201 (8, 3) against 262, 160 columns 373 (16, 3) against 431; 64^3, 13 points, FP64, 96
+    // columns 194 (16, 3) against 220). Wider rows: panels of (16, 2) where they fill their
+    // lanes (256 columns 544 against 574), else of (16, 1) with a whole short row in flight
+    // (320 columns, 128^3: 1.67 against 1.80 ms). FP64 rows of 9 to 16 and 25 to 32 vectors
+    // do as well or better in (16, 1) panels.
+    const int lanes16 = (nvec + 15) / 16 * 16, lanes32 = (nvec + 31) / 32 * 32;
+    const int lanes24 = (nvec + 23) / 24 * 24;
+    const bool f64 = sizeof(T) == 8;
+    // 0: (8, 1), 1: (8, 2), 2: (8, 3), 3: (16, 1), 4: (16, 2), 5: (16, 3), 6: (32, 3)
+    int shape = 3;
+    if (nvec <= 8) shape = 0;
+    else if (nvec <= 16) shape = f64 && k <= 8 ? 3 : 1;
+    else if (nvec <= 24) shape = 2;
+    else if (nvec <= 32) shape = f64 && k <= 8 ? 3 : 4;
+    else if (nvec <= 48) shape = 5;
+    else if (k > 8 && k <= 16 && nvec > 64 && nvec <= 96) shape = 6;
+    else if (lanes32 * 19 <= lanes16 * 20) shape = f64 && k <= 8 ? 3 : 4;
+    else if (lanes24 < lanes16) shape = 2;
+    if (k > 16 && shape < 3) shape = nvec <= 16 ? 3 : 4;  // 8 lanes hold 16 entries
+#define FE_SHAPES(CORR_)                                          \
+  do {                                                            \
+    if (k <= 8) {                                                 \
+      if (shape == 0) FE_ROWS(V16, 8, 1, 1, 7, CORR_);            \
+      if (shape == 1) FE_ROWS(V16, 8, 2, 1, 2, CORR_);            \
+      if (shape == 2) FE_ROWS(V16, 8, 3, 1, 2, CORR_);            \
+      if (shape == 3) FE_ROWS(V16, 16, 1, 1, 7, CORR_);           \
+      if (shape == 4) FE_ROWS(V16, 16, 2, 1, 2, CORR_);           \
+      FE_ROWS(V16, 16, 3, 1, 2, CORR_);                           \
+    }                                                             \
+    if (k <= 16) {                                                \
+      if (shape == 0) FE_ROWS_F(V16, 8, 1, 2, 4, false, CORR_);   \
+      if (shape == 1) FE_ROWS_F(V16, 8, 2, 2, 2, false, CORR_);   \
+      if (shape == 2) FE_ROWS_F(V16, 8, 3, 2, 2, false, CORR_);   \
+      if (shape == 3) FE_ROWS_F(V16, 16, 1, 1, 13, false, CORR_); \
+      if (shape == 4) FE_ROWS_F(V16, 16, 2, 1, 2, false, CORR_);  \
+      if (shape == 6) FE_ROWS_F(V16, 32, 3, 1, 2, false, CORR_);  \
+      FE_ROWS_F(V16, 16, 3, 1, 2, false, CORR_);                  \
+    }                                                             \
+    if (shape == 3) FE_ROWS_F(V16, 16, 1, 2, 8, false, CORR_);    \
+    if (shape == 4) FE_ROWS_F(V16, 16, 2, 2, 2, false, CORR_);    \
+    FE_ROWS_F(V16, 16, 3, 2, 2, false, CORR_);                    \
+  } while (0)
     if constexpr (sizeof(T) == 4) {
-      if (R) {
-        if (narrow && k <= 8) FE_ROWS(V16, 8, 1, 1, 7, true);
-        if (narrow) FE_ROWS_F(V16, 8, 1, 2, 4, false, true);
-        if (k <= 8) FE_ROWS(V16, 16, 1, 1, 7, true);
-        if (k <= 16) FE_ROWS_F(V16, 16, 1, 1, 4, false, true);
-        FE_ROWS_F(V16, 16, 1, 2, 8, false, true);
-      }
+      if (R) FE_SHAPES(true);
     }
-    if (narrow && k <= 8) FE_ROWS(V16, 8, 1, 1, 7, false);
-    if (narrow) FE_ROWS_F(V16, 8, 1, 2, 4, false, false);
-    if (k <= 8) FE_ROWS(V16, 16, 1, 1, 7, false);
-    if (k <= 16) FE_ROWS_F(V16, 16, 1, 1, 4, false, false);
-    FE_ROWS_F(V16, 16, 1, 2, 8, false, false);
+    FE_SHAPES(false);
+#undef FE_SHAPES
   }
   if constexpr (sizeof(T) == 4) {
-    if (vec == 2) {
-      if (k <= 16) FE_ROWS(2, 16, 2, 1, 4, false);
-      FE_ROWS_F(2, 16, 2, 2, 4, false, false);
-    }
+    if (vec == 2) FE_ROWS(2, 16, 2, 1, 4, false);
+  } else {
+    FE_ROWS(1, 16, 3, 1, 4, false);  // FP64 rows that start at any element
   }
-  // rows that start at any element: up to three elements a lane
-  if (nvec <= 16 && k <= 16) FE_ROWS_F(1, 16, 1, 1, 4, false, false);
-  if (nvec <= 32 && k <= 16) FE_ROWS(1, 16, 2, 1, 4, false);
-  if (k <= 16) FE_ROWS(1, 16, 3, 1, 4, false);
-  FE_ROWS_F(1, 16, 3, 2, 4, false, false);
+  return false;
 #undef FE_ROWS_F
 #undef FE_ROWS
 }
