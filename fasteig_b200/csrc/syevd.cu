@@ -4,8 +4,9 @@
 // host Eigen SelfAdjointEigenSolver of its CPU path (src/core/RitzExtraction.cpp:104).
 //
 // Four kernels, each batched over matrices (matrix p: A + p*lda*lda, size m[p]):
-//   1. sytrd: Householder tridiagonalization, one cluster of 8 CTAs per matrix while
-//      the matrix fits their shared memory (k <= 469), else one CTA. Step j reflects
+//   1. sytrd: Householder tridiagonalization, one CTA per matrix in shared memory up to
+//      k = 128, one cluster of 8 CTAs while the matrix fits their shared memory
+//      (k <= 469), else one CTA. Step j reflects
 //      column j below the diagonal (dlarfg convention: beta = -sign(alpha)||x||,
 //      tau = (beta - alpha)/beta, v = x/(alpha - beta), v0 = 1), then
 //      p = tau A22 v, w = p - (tau/2)(p.v) v, A22 -= v w^T + w v^T (both triangles
@@ -163,6 +164,118 @@ sytrd_kernel(const int32_t* __restrict__ msz, double* __restrict__ A, int64_t ld
       dp[0] = M[0];
     }
   }
+}
+
+// Householder tridiagonalization of matrices of up to kTrdSmall rows, one CTA each, with the
+// same steps as sytrd_kernel. A step is a chain of short reductions, so what bounds it is
+// the number of barriers: every warp forms the reflector for itself from the column in
+// shared memory (a lane holds rows lane, lane + 32, ...), which leaves two, one before and
+// one after w is complete (36 rows: 50 us, 96 rows 183 us; 89 and 264 us with the cluster
+// kernel's two cluster barriers a step).
+constexpr int kTrdSmall = 128;
+
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS)
+sytrd_small_kernel(const int32_t* __restrict__ msz, double* __restrict__ A, int64_t lda,
+                   double* __restrict__ d, double* __restrict__ e, double* __restrict__ tau,
+                   int64_t vec_stride) {
+  constexpr int U = kTrdSmall / 32, WARPS = THREADS / 32;
+  extern __shared__ double sh[];
+  const int p = blockIdx.x;
+  const int k = msz[p];
+  const int ld = k + 1;
+  double* Ap = A + static_cast<int64_t>(p) * lda * lda;
+  double* dp = d + p * vec_stride;
+  double* ep = e + p * vec_stride;
+  double* tp = tau + p * vec_stride;
+  double* S = sh;            // column-major, ld
+  double* w = sh + k * ld;   // tau A22 v
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  for (int c = warp; c < k; c += WARPS)
+    for (int r = lane; r < k; r += 32) S[c * ld + r] = Ap[c * lda + r];
+  __syncthreads();
+  auto warp_total = [](double v) {
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+  };
+  for (int j = 0; j + 2 < k; ++j) {
+    const int m = k - j - 1;  // rows of A22 = A(j+1:, j+1:)
+    const double* col = S + j * ld + j + 1;
+    double v[U], part = 0.0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = lane + 32 * u;
+      v[u] = i < m ? col[i] : 0.0;
+      if (i > 0) part = fma(v[u], v[u], part);
+    }
+    const double xn2 = warp_total(part);
+    const double alpha = col[0];
+    double beta = alpha, t = 0.0, sc = 0.0;
+    if (xn2 != 0.0) {
+      beta = -copysign(sqrt(alpha * alpha + xn2), alpha);
+      t = (beta - alpha) / beta;
+      sc = 1.0 / (alpha - beta);
+    }
+    if (tid == 0) {
+      dp[j] = S[j * ld + j];
+      ep[j] = beta;
+      tp[j] = t;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = lane + 32 * u;
+      v[u] = i == 0 ? 1.0 : v[u] * sc;
+      if (warp == 0 && i < m) Ap[j * lda + j + 1 + i] = v[u];  // for the back-transformation
+    }
+    if (t == 0.0) continue;  // the same in every thread
+    double* T = S + (j + 1) * ld + j + 1;  // A22
+    for (int c = warp; c < m; c += WARPS) {
+      double acc = 0.0;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = lane + 32 * u;
+        if (i < m) acc = fma(T[c * ld + i], v[u], acc);
+      }
+      acc = warp_total(acc);
+      if (lane == 0) w[c] = t * acc;
+    }
+    __syncthreads();
+    double wr[U], pv = 0.0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = lane + 32 * u;
+      wr[u] = i < m ? w[i] : 0.0;
+      pv = fma(wr[u], v[u], pv);
+    }
+    const double K = 0.5 * t * warp_total(pv);
+#pragma unroll
+    for (int u = 0; u < U; ++u) wr[u] = fma(-K, v[u], wr[u]);
+    for (int c = warp; c < m; c += WARPS) {
+      const double vc = c == 0 ? 1.0 : col[c] * sc;
+      const double wc = fma(-K, vc, w[c]);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = lane + 32 * u;
+        if (i < m) T[c * ld + i] -= v[u] * wc + wr[u] * vc;
+      }
+    }
+    __syncthreads();
+  }
+  if (tid == 0) {
+    if (k >= 2) {
+      const double* c = S + (k - 2) * ld + k - 2;
+      dp[k - 2] = c[0];
+      ep[k - 2] = c[1];
+      tp[k - 2] = 0.0;
+      dp[k - 1] = c[ld + 1];
+    } else if (k == 1) {
+      dp[0] = S[0];
+    }
+  }
+}
+
+size_t sytrd_small_smem(int kmax) {
+  return (static_cast<size_t>(kmax) * (kmax + 1) + kmax) * sizeof(double);
 }
 
 // Householder tridiagonalization on a cluster of kClu CTAs with the whole matrix in
@@ -409,18 +522,23 @@ __device__ __forceinline__ double hash_uniform(uint64_t a, uint64_t b) {
   return static_cast<double>(z >> 11) * (2.0 / 9007199254740992.0) - 1.0;
 }
 
-// LU of T - lambda I with partial pivoting (one thread). U: reciprocal diagonal u0
-// (pivots smaller than `tiny` replaced by +-tiny first), first and second
-// superdiagonals u1, u2 (zero past the end); L multipliers l; piv[i] = 1 where rows
+// LU of T - lambda I with partial pivoting (one thread), U scaled by its reciprocal
+// diagonal so that a back substitution step is one dependent multiply-add: u0 = 1 / u_ii
+// (pivots smaller than `tiny` replaced by +-tiny first), u1, u2 the first and second
+// superdiagonals times u0 (zero past the end); L multipliers l; piv[i] = 1 where rows
 // i, i+1 were swapped.
-__device__ void tri_factor(const double* d, const double* e, int k, double lam, double tiny,
-                           double* u0, double* u1, double* u2, double* l, double* piv) {
+__device__ __forceinline__ void tri_factor(const double* __restrict__ d,
+                                           const double* __restrict__ e, int k, double lam,
+                                           double tiny, double* __restrict__ u0,
+                                           double* __restrict__ u1, double* __restrict__ u2,
+                                           double* __restrict__ l, double* __restrict__ piv) {
   auto inv_pivot = [tiny](double pv) {
     if (fabs(pv) < tiny) pv = (pv != 0.0) ? copysign(tiny, pv) : tiny;
     return 1.0 / pv;
   };
   double cur_d = d[0] - lam;
   double cur_u = k > 1 ? e[0] : 0.0;
+#pragma unroll 2
   for (int i = 0; i + 1 < k; ++i) {
     const double sub = e[i];
     const double nd = d[i + 1] - lam;
@@ -430,8 +548,9 @@ __device__ void tri_factor(const double* d, const double* e, int k, double lam, 
       if (cur_d == 0.0) cur_d = tiny;
       const double mlt = sub / cur_d;
       l[i] = mlt;
-      u0[i] = inv_pivot(cur_d);
-      u1[i] = cur_u;
+      const double r = inv_pivot(cur_d);
+      u0[i] = r;
+      u1[i] = cur_u * r;
       u2[i] = 0.0;
       cur_d = nd - mlt * cur_u;
       cur_u = nu;
@@ -439,9 +558,10 @@ __device__ void tri_factor(const double* d, const double* e, int k, double lam, 
       piv[i] = 1.0;
       const double mlt = cur_d / sub;
       l[i] = mlt;
-      u0[i] = inv_pivot(sub);
-      u1[i] = nd;
-      u2[i] = nu;
+      const double r = inv_pivot(sub);
+      u0[i] = r;
+      u1[i] = nd * r;
+      u2[i] = i + 2 < k ? nu * r : 0.0;
       cur_d = cur_u - mlt * nd;
       cur_u = -mlt * nu;
     }
@@ -449,30 +569,31 @@ __device__ void tri_factor(const double* d, const double* e, int k, double lam, 
   u0[k - 1] = inv_pivot(cur_d);
   u1[k - 1] = 0.0;
   u2[k - 1] = 0.0;
-  if (k >= 2) u2[k - 2] = 0.0;
 }
 
 // x <- (T - lambda I)^{-1} x with the factors above (one thread). The running values
-// stay in registers, so each step's chain is a few FMAs and no load waits on a store.
-__device__ void tri_solve(int k, const double* u0, const double* u1, const double* u2,
-                          const double* l, const double* piv, double* x) {
+// stay in registers, so each step's chain is one multiply-add and no load waits on a store.
+__device__ __forceinline__ void tri_solve(int k, const double* __restrict__ u0,
+                                          const double* __restrict__ u1,
+                                          const double* __restrict__ u2,
+                                          const double* __restrict__ l,
+                                          const double* __restrict__ piv,
+                                          double* __restrict__ x) {
   double xi = x[0];
+#pragma unroll 8
   for (int i = 0; i + 1 < k; ++i) {
     const double xn = x[i + 1];
     const double li = l[i];
-    if (piv[i] != 0.0) {
-      x[i] = xn;
-      xi = xi - li * xn;
-    } else {
-      x[i] = xi;
-      xi = xn - li * xi;
-    }
+    const bool swap = piv[i] != 0.0;
+    const double a = swap ? xn : xi, b = swap ? xi : xn;
+    x[i] = a;
+    xi = fma(-li, a, b);
   }
   x[k - 1] = xi;
   double x1 = 0.0, x2 = 0.0;  // x[i + 1], x[i + 2]
+#pragma unroll 8
   for (int i = k - 1; i >= 0; --i) {
-    const double s = x[i] - u1[i] * x1 - u2[i] * x2;
-    const double r = s * u0[i];
+    const double r = fma(-u1[i], x1, fma(-u2[i], x2, x[i] * u0[i]));
     x[i] = r;
     x2 = x1;
     x1 = r;
@@ -485,7 +606,10 @@ __device__ __forceinline__ double warp_sum(double v) {
 }
 
 // One warp per cluster start: eigenvectors of tridiagonal p into Z_T (column-major,
-// ldz) for the cluster's eigenvalues. Scratch: 6 k doubles per eigenvalue index.
+// ldz) for the cluster's eigenvalues. Scratch: 6 k doubles per eigenvalue index, in shared
+// memory (SMEM; 6 k per warp) or, past its size, in `scratch`. One thread runs the factor
+// and the solves, so the time is the chain of its loads and operations.
+template <bool SMEM>
 __global__ void stein_kernel(const int32_t* __restrict__ msz, const double* __restrict__ d,
                              const double* __restrict__ e, int64_t vec_stride,
                              const double* __restrict__ W, int64_t ldw,
@@ -509,7 +633,9 @@ __global__ void stein_kernel(const int32_t* __restrict__ msz, const double* __re
   if (t0 > 0 && wp[t0] - wp[t0 - 1] <= gap) return;  // not the first of its cluster
   int t1 = t0;
   while (t1 + 1 < k && wp[t1 + 1] - wp[t1] <= gap) ++t1;
-  double* s = scratch + (static_cast<int64_t>(p) * ldz + t0) * scratch_stride;
+  extern __shared__ double stein_sh[];
+  double* s = SMEM ? stein_sh + (threadIdx.x / 32) * 6 * k
+                   : scratch + (static_cast<int64_t>(p) * ldz + t0) * scratch_stride;
   double *u0 = s, *u1 = s + k, *u2 = s + 2 * k, *l = s + 3 * k, *piv = s + 4 * k, *x = s + 5 * k;
   const double tiny = kEps * fmax(tnorm, kTiny);
   for (int t = t0; t <= t1; ++t) {
@@ -679,7 +805,7 @@ int current_device() {
 // cudaFuncSetAttribute(MaxDynamicSharedMemorySize) once per (kernel slot, device).
 void set_max_smem_once(const void* kernel, int bytes, int dev, int slot) {
   static std::mutex mu;
-  static bool done[4][64] = {};
+  static bool done[5][64] = {};
   std::lock_guard<std::mutex> lock(mu);
   const bool tracked = dev >= 0 && dev < 64;
   if (tracked && done[slot][dev]) return;
@@ -767,7 +893,19 @@ void syevd_batched_prepared(int count, int kmax, const SyevdWs& w, double* A, in
   FE_CHECK_CUDA(cudaMemsetAsync(info, 0, sizeof(int32_t) * count, s));
   const int optin = smem_optin();
   const int dev = current_device();
-  if (use_cluster_sytrd(kmax, optin, dev)) {
+  if (g_sytrd_mode == 0 && kmax <= kTrdSmall) {
+    const size_t smem = sytrd_small_smem(kmax);
+    if (kmax <= 48) {
+      sytrd_small_kernel<256><<<count, 256, smem, s>>>(w.msz, A, lda, w.d, w.e, w.tau,
+                                                       w.vec_stride);
+    } else {
+      set_max_smem_once(reinterpret_cast<const void*>(sytrd_small_kernel<512>), optin - 256, dev,
+                        4);
+      sytrd_small_kernel<512><<<count, 512, smem, s>>>(w.msz, A, lda, w.d, w.e, w.tau,
+                                                       w.vec_stride);
+    }
+    check_launch("sytrd_small_kernel");
+  } else if (use_cluster_sytrd(kmax, optin, dev)) {
     sytrd_cluster_kernel<<<count * kClu, kCluThreads, sytrd_cluster_smem(kmax), s>>>(
         w.msz, A, lda, w.d, w.e, w.tau, w.vec_stride, kmax);
     check_launch("sytrd_cluster_kernel");
@@ -785,9 +923,17 @@ void syevd_batched_prepared(int count, int kmax, const SyevdWs& w, double* A, in
                                                             lda, w.tnorm, info);
   check_launch("stebz_kernel");
   FE_CHECK_CUDA(cudaMemsetAsync(Z, 0, sizeof(double) * count * lda * lda, s));
-  stein_kernel<<<dim3((kmax + 3) / 4, count), 128, 0, s>>>(w.msz, w.d, w.e, w.vec_stride, W, lda,
+  const size_t stein_smem = size_t(4) * 6 * kmax * sizeof(double);
+  const dim3 stein_grid((kmax + 3) / 4, count);
+  if (stein_smem + 1024 <= static_cast<size_t>(optin)) {
+    set_max_smem_once(reinterpret_cast<const void*>(stein_kernel<true>), optin - 256, dev, 3);
+    stein_kernel<true><<<stein_grid, 128, stein_smem, s>>>(w.msz, w.d, w.e, w.vec_stride, W, lda,
                                                            w.tnorm, Z, lda, w.scratch,
                                                            w.scratch_stride);
+  } else {
+    stein_kernel<false><<<stein_grid, 128, 0, s>>>(w.msz, w.d, w.e, w.vec_stride, W, lda, w.tnorm,
+                                                   Z, lda, w.scratch, w.scratch_stride);
+  }
   check_launch("stein_kernel");
   const size_t orm_smem = ormtr_smem_bytes(kmax);
   if (orm_smem + 1024 <= static_cast<size_t>(optin)) {
