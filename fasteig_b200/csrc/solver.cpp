@@ -1661,15 +1661,12 @@ struct GenBlockOpsT {
   // are dropped as noise: about sqrt(unit roundoff) of the block's precision.
   static constexpr double kRankFloor = sizeof(T) == 4 ? 1e-3 : 1e-7;
 
+  // Without a mass matrix the B blocks are the blocks themselves (the callers alias them):
+  // every product, rotation and copy of a B block that is not there is skipped.
   void bapply(const T* X, T* BX, int64_t cols) {
-    if (cols <= 0) return;
-    if (B) {
-      csr_spmm<T>(*B, X, ld, BX, ld, nullptr, 0, cols, 1.0, 0.0, 0.0, ctx.stream);
-      st.spmm_launches += 1;
-    } else {
-      FE_CHECK_CUDA(cudaMemcpy2DAsync(BX, ld * sizeof(T), X, ld * sizeof(T), cols * sizeof(T), n,
-                                      cudaMemcpyDeviceToDevice, ctx.stream));
-    }
+    if (cols <= 0 || !B) return;
+    csr_spmm<T>(*B, X, ld, BX, ld, nullptr, 0, cols, 1.0, 0.0, 0.0, ctx.stream);
+    st.spmm_launches += 1;
   }
   void happly(const T* X, T* AX, int64_t cols) {
     if (cols <= 0) return;
@@ -1697,10 +1694,25 @@ struct GenBlockOpsT {
     std::vector<double> norms, w, inv;
     for (int pass = 0; pass < 2; ++pass) {
       bapply(cur, tmpB, cols);
-      residual_norms<T>(nullptr, cur, tmpB, ld, n, cols, nullptr, nullptr, 0, nullptr,
+      residual_norms<T>(nullptr, cur, B ? tmpB : cur, ld, n, cols, nullptr, nullptr, 0, nullptr,
                              sm.xnorm.as<double>(), nullptr, sm.rws.get(), sm.rws.bytes(), s, 2);
+      copy(tmp, cur, cols);
+      double* G = sm.G.as<double>();
+      if (k > 0) {
+        for (int g = 0; g < 2; ++g) {
+          gram_block<T>(sm, V, ld, tmpB, ld, n, k, cols, G, s);
+          rotate_block<T>(sm, V, ld, G, tmp, ld, n, k, cols, -1.0, 1.0, s);
+          if (B) rotate_block<T>(sm, BV, ld, G, tmpB, ld, n, k, cols, -1.0, 1.0, s);
+        }
+      }
+      gram_block<T>(sm, tmp, ld, tmpB, ld, n, cols, cols, G, s);
+      symmetrize(G, cols, sm.cap, s);
+      eig.run(G, cols, sm.cap, sm.W.as<double>());
+      // one wait for the norms and the eigenvalues
       norms.resize(cols);
+      w.resize(cols);
       ctx.to_host(norms.data(), sm.xnorm.as<double>(), cols);
+      ctx.to_host(w.data(), sm.W.as<double>(), cols);
       ctx.sync();
       double scale = 0.0;
       for (double v : norms) {
@@ -1709,21 +1721,6 @@ struct GenBlockOpsT {
         scale = std::max(scale, v);
       }
       if (scale == 0.0) return 0;
-      copy(tmp, cur, cols);
-      double* G = sm.G.as<double>();
-      if (k > 0) {
-        for (int g = 0; g < 2; ++g) {
-          gram_block<T>(sm, V, ld, tmpB, ld, n, k, cols, G, s);
-          rotate_block<T>(sm, V, ld, G, tmp, ld, n, k, cols, -1.0, 1.0, s);
-          rotate_block<T>(sm, BV, ld, G, tmpB, ld, n, k, cols, -1.0, 1.0, s);
-        }
-      }
-      gram_block<T>(sm, tmp, ld, tmpB, ld, n, cols, cols, G, s);
-      symmetrize(G, cols, sm.cap, s);
-      eig.run(G, cols, sm.cap, sm.W.as<double>());
-      w.resize(cols);
-      ctx.to_host(w.data(), sm.W.as<double>(), cols);
-      ctx.sync();
       const double smax = std::sqrt(std::max(w[cols - 1], 0.0));
       const int64_t capacity = std::min<int64_t>(cols, n - k);
       const double cut = std::max(rank_tol * scale, kRankFloor * smax);
@@ -1745,10 +1742,10 @@ struct GenBlockOpsT {
       ctx.to_device(ds, inv.data(), rank);
       small_gather_scale(G, sm.cap, cols, di, ds, rank, sm.Rinv.as<double>(), sm.cap, s);
       rotate_block<T>(sm, tmp, ld, sm.Rinv.as<double>(), out, ld, n, cols, rank, 1.0, 0.0, s);
-      rotate_block<T>(sm, tmpB, ld, sm.Rinv.as<double>(), Bout, ld, n, cols, rank, 1.0, 0.0, s);
+      if (B)
+        rotate_block<T>(sm, tmpB, ld, sm.Rinv.as<double>(), Bout, ld, n, cols, rank, 1.0, 0.0, s);
       cur = out;
       cols = rank;
-      ctx.sync();
     }
     return rank;
   }
@@ -1767,8 +1764,9 @@ struct GenBlockOpsT {
     ctx.sync();
     if (info != 0) throw Error(FE_ERR_NOT_SPD, std::string(what) + ": weighted QR failed.");
     rotate_block<T>(sm, X, ld, sm.Rinv.as<double>(), tmp, ld, n, b, b, 1.0, 0.0, s);
-    rotate_block<T>(sm, BX, ld, sm.Rinv.as<double>(), tmpB, ld, n, b, b, 1.0, 0.0, s);
     copy(X, tmp, b);
+    if (!B) return;
+    rotate_block<T>(sm, BX, ld, sm.Rinv.as<double>(), tmpB, ld, n, b, b, 1.0, 0.0, s);
     copy(BX, tmpB, b);
   }
 };
@@ -1778,8 +1776,11 @@ using GenBlockOps = GenBlockOpsT<double>;
 template <typename T>
 struct LobpcgBlocks {
   Block<T> X, AX, BX, R, Pd, S, AS, BS, T1, T2, Wsrc;
-  void allocate(int64_t n, int64_t cap) {
-    for (Block<T>* q : {&X, &AX, &BX, &R, &Pd, &S, &AS, &BS, &T1, &T2, &Wsrc}) q->allocate(n, cap);
+  // The B blocks (and the scratch that goes with them) only with a mass matrix.
+  void allocate(int64_t n, int64_t cap, bool with_b) {
+    for (Block<T>* q : {&X, &AX, &R, &Pd, &S, &AS, &T1, &Wsrc}) q->allocate(n, cap);
+    if (with_b)
+      for (Block<T>* q : {&BX, &BS, &T2}) q->allocate(n, cap);
   }
 };
 
@@ -1800,17 +1801,21 @@ void lobpcg_gen_phase(Context& ctx, SmallState& sm, ProjectedEig& eig, const Csr
   cudaStream_t s = ctx.stream;
   const int64_t n = A.rows, nev = opt.nev, ld = L.X.ld;
   GenBlockOpsT<T> g{ctx, sm, eig, A, B, sign, n, ld, st, DeviceBuffer(64)};
-  if (g.ortho(nullptr, nullptr, 0, L.X.data(), b, L.X.data(), L.BX.data(), L.T1.data(),
-              L.T2.data()) < b)
+  // without a mass matrix the B blocks are the blocks themselves
+  T* const BX = B ? L.BX.data() : L.X.data();
+  T* const BS = B ? L.BS.data() : L.S.data();
+  T* const T2 = B ? L.T2.data() : L.T1.data();
+  if (g.ortho(nullptr, nullptr, 0, L.X.data(), b, L.X.data(), BX, L.T1.data(),
+              T2) < b)
     throw Error(FE_ERR_NOT_SPD, "LOBPCGSolver: initial block is rank deficient.");
   g.happly(L.X.data(), L.AX.data(), b);
   g.copy(L.S.data(), L.X.data(), b);
   g.copy(L.AS.data(), L.AX.data(), b);
-  g.copy(L.BS.data(), L.BX.data(), b);
+  if (B) g.copy(BS, BX, b);
   gram_block<T>(sm, L.S.data(), ld, L.AS.data(), ld, n, b, b, sm.G.as<double>(), s);
   ritz_extract<T>(ctx, sm, eig, sm.G.as<double>(), L.S.data(), L.AS.data(), ld, n, b, b, "sr",
                   L.X.data(), L.AX.data(), L.R.data(), coef.as<double>(), g.idx_dev, ritz,
-                  L.BS.data(), L.BX.data());
+                  B ? BS : nullptr, B ? BX : nullptr);
   auto worst_nev = [&] {
     double w = 0;
     for (int64_t j = 0; j < nev; ++j) w = std::max(w, ritz.rel[j]);
@@ -1832,24 +1837,24 @@ void lobpcg_gen_phase(Context& ctx, SmallState& sm, ProjectedEig& eig, const Csr
     const int64_t na = static_cast<int64_t>(active.size());
     ctx.to_device(act.as<int32_t>(), active.data(), na);
     gather_columns<T>(L.R.data(), ld, act.as<int32_t>(), na, L.Wsrc.data(), ld, n, s, t);
-    g.bcholqr(L.X.data(), L.BX.data(), b, L.T1.data(), L.T2.data(), "LOBPCGSolver: Ritz-vector");
+    g.bcholqr(L.X.data(), BX, b, L.T1.data(), T2, "LOBPCGSolver: Ritz-vector");
     g.copy(L.S.data(), L.X.data(), b);
-    g.copy(L.BS.data(), L.BX.data(), b);
+    if (B) g.copy(BS, BX, b);
     int64_t cols = b;
-    const int64_t rw = g.ortho(L.S.data(), L.BS.data(), cols, L.Wsrc.data(), na, L.S.col(cols),
-                               L.BS.col(cols), L.T1.data(), L.T2.data());
+    const int64_t rw = g.ortho(L.S.data(), BS, cols, L.Wsrc.data(), na, L.S.col(cols),
+                               BS + cols, L.T1.data(), T2);
     cols += std::min(rw, cap - cols);
     if (have_p && cols < cap) {
       gather_columns<T>(L.Pd.data(), ld, act.as<int32_t>(), na, L.Wsrc.data(), ld, n, s);
-      const int64_t rp = g.ortho(L.S.data(), L.BS.data(), cols, L.Wsrc.data(), na, L.S.col(cols),
-                                 L.BS.col(cols), L.T1.data(), L.T2.data());
+      const int64_t rp = g.ortho(L.S.data(), BS, cols, L.Wsrc.data(), na, L.S.col(cols),
+                                 BS + cols, L.T1.data(), T2);
       cols += std::min(rp, cap - cols);
     }
     g.happly(L.S.data(), L.AS.data(), cols);
     gram_block<T>(sm, L.S.data(), ld, L.AS.data(), ld, n, cols, cols, sm.G.as<double>(), s);
     ritz_extract<T>(ctx, sm, eig, sm.G.as<double>(), L.S.data(), L.AS.data(), ld, n, cols, b, "sr",
                     L.X.data(), L.AX.data(), L.R.data(), coef.as<double>(), g.idx_dev, ritz,
-                    L.BS.data(), L.BX.data());
+                    B ? BS : nullptr, B ? BX : nullptr);
     // P = S C with the X rows of C zeroed.
     FE_CHECK_CUDA(cudaMemset2DAsync(coef.get(), cap * 8, 0, b * 8, b, s));
     rotate_block<T>(sm, L.S.data(), ld, coef.as<double>(), L.Pd.data(), ld, n, cols, b, 1.0, 0.0,
@@ -1902,7 +1907,7 @@ void lobpcg_gen_solve(const Csr& A, const Csr* B, const Options& opt, double* ei
   LobpcgBlocks<double> D;
   if (mixed) {
     LobpcgBlocks<float> F;
-    F.allocate(n, cap);
+    F.allocate(n, cap, B != nullptr);
     {
       Block<double> X0;
       X0.allocate(n, b);
@@ -1913,11 +1918,11 @@ void lobpcg_gen_solve(const Csr& A, const Csr* B, const Options& opt, double* ei
     lobpcg_gen_phase<float>(ctx, sm, eig, A, B, opt, sign, b, cap, t, F, ritz, it_done,
                             std::max(tol, opt.mixed_switch), true, act, coef, st);
     st.fp32_iterations = static_cast<double>(it_done);
-    D.allocate(n, cap);
+    D.allocate(n, cap, B != nullptr);
     convert<float, double>(F.X.data(), F.X.ld, D.X.data(), D.X.ld, n, b, s);
     ctx.sync();
   } else {
-    D.allocate(n, cap);
+    D.allocate(n, cap, B != nullptr);
     fill_initial_block(ctx, D.X.data(), D.X.ld, n, b, opt.seed_or_default(), opt.init == "host");
   }
   const int64_t it64 = it_done;
@@ -1932,8 +1937,10 @@ void lobpcg_gen_solve(const Csr& A, const Csr* B, const Options& opt, double* ei
 template <typename T>
 struct DavidsonBlocks {
   Block<T> V, AV, BV, X, AX, BX, R, T1, T2, Wsrc;
-  void allocate(int64_t n, int64_t cap) {
-    for (Block<T>* q : {&V, &AV, &BV, &X, &AX, &BX, &R, &T1, &T2, &Wsrc}) q->allocate(n, cap);
+  void allocate(int64_t n, int64_t cap, bool with_b) {
+    for (Block<T>* q : {&V, &AV, &X, &AX, &R, &T1, &Wsrc}) q->allocate(n, cap);
+    if (with_b)
+      for (Block<T>* q : {&BV, &BX, &T2}) q->allocate(n, cap);
   }
 };
 
@@ -1954,6 +1961,10 @@ void davidson_gen_phase(Context& ctx, SmallState& sm, ProjectedEig& eig, const C
   const int64_t n = A.rows, nev = opt.nev, ld = L.V.ld;
   const std::string which = opt.which;
   GenBlockOpsT<T> g{ctx, sm, eig, A, B, 1.0, n, ld, st, DeviceBuffer(64)};
+  // without a mass matrix the B blocks are the blocks themselves
+  T* const BX = B ? L.BX.data() : L.X.data();
+  T* const BV = B ? L.BV.data() : L.V.data();
+  T* const T2 = B ? L.T2.data() : L.T1.data();
   double* Pm = proj.as<double>();
   double* Pw = sm.G.as<double>();
   auto extract = [&](int64_t cols) {
@@ -1961,21 +1972,21 @@ void davidson_gen_phase(Context& ctx, SmallState& sm, ProjectedEig& eig, const C
                                     cudaMemcpyDeviceToDevice, s));
     ritz_extract<T>(ctx, sm, eig, Pw, L.V.data(), L.AV.data(), ld, n, cols, bw, which,
                     L.X.data(), L.AX.data(), L.R.data(), coef.as<double>(), g.idx_dev, ritz,
-                    L.BV.data(), L.BX.data());
+                    B ? BV : nullptr, B ? BX : nullptr);
   };
-  if (g.ortho(nullptr, nullptr, 0, L.X.data(), bw, L.X.data(), L.BX.data(), L.T1.data(),
-              L.T2.data()) < bw)
+  if (g.ortho(nullptr, nullptr, 0, L.X.data(), bw, L.X.data(), BX, L.T1.data(),
+              T2) < bw)
     throw Error(FE_ERR_NOT_SPD, "DavidsonSolver: initial block is rank deficient.");
   g.copy(L.V.data(), L.X.data(), bw);
-  g.copy(L.BV.data(), L.BX.data(), bw);
+  if (B) g.copy(BV, BX, bw);
   g.happly(L.V.data(), L.AV.data(), bw);
   gram_block<T>(sm, L.V.data(), ld, L.AV.data(), ld, n, bw, bw, Pm, s);
   extract(bw);
   std::vector<double> history;
   while (it_done < opt.maxiter) {
-    g.bcholqr(L.X.data(), L.BX.data(), bw, L.T1.data(), L.T2.data(), "DavidsonSolver: restart");
+    g.bcholqr(L.X.data(), BX, bw, L.T1.data(), T2, "DavidsonSolver: restart");
     g.copy(L.V.data(), L.X.data(), bw);
-    g.copy(L.BV.data(), L.BX.data(), bw);
+    if (B) g.copy(BV, BX, bw);
     g.happly(L.V.data(), L.AV.data(), bw);
     FE_CHECK_CUDA(cudaMemset2DAsync(Pm, cap * 8, 0, cap * 8, cap, s));
     gram_block<T>(sm, L.V.data(), ld, L.AV.data(), ld, n, bw, bw, Pm, s);
@@ -1989,8 +2000,8 @@ void davidson_gen_phase(Context& ctx, SmallState& sm, ProjectedEig& eig, const C
       if (cc == 0 || cols + cc > cap) break;
       ctx.to_device(act.as<int32_t>(), active.data(), cc);
       gather_columns<T>(L.R.data(), ld, act.as<int32_t>(), cc, L.Wsrc.data(), ld, n, s, t);
-      const int64_t r = g.ortho(L.V.data(), L.BV.data(), cols, L.Wsrc.data(), cc, L.V.col(cols),
-                                L.BV.col(cols), L.T1.data(), L.T2.data());
+      const int64_t r = g.ortho(L.V.data(), BV, cols, L.Wsrc.data(), cc, L.V.col(cols),
+                                BV + cols, L.T1.data(), T2);
       if (r == 0) break;
       g.happly(L.V.col(cols), L.AV.col(cols), r);
       // projected[:cols, cols:cols+r] = V^T A W, mirrored; diagonal block W^T A W.
@@ -2057,7 +2068,7 @@ void davidson_gen_solve(const Csr& A, const Csr* B, const Options& opt, double* 
   DavidsonBlocks<double> D;
   if (mixed) {
     DavidsonBlocks<float> F;
-    F.allocate(n, cap);
+    F.allocate(n, cap, B != nullptr);
     {
       Block<double> X0;
       X0.allocate(n, bw);
@@ -2069,11 +2080,11 @@ void davidson_gen_solve(const Csr& A, const Csr* B, const Options& opt, double* 
     davidson_gen_phase<float>(ctx, sm, eig, A, B, opt, bw, cap, t, F, ritz, it_done, floor32,
                               floor32, true, act, coef, proj, st);
     st.fp32_iterations = static_cast<double>(it_done);
-    D.allocate(n, cap);
+    D.allocate(n, cap, B != nullptr);
     convert<float, double>(F.X.data(), F.X.ld, D.X.data(), D.X.ld, n, bw, s);
     ctx.sync();
   } else {
-    D.allocate(n, cap);
+    D.allocate(n, cap, B != nullptr);
     fill_initial_block(ctx, D.X.data(), D.X.ld, n, bw, opt.seed_or_default(), opt.init == "host");
   }
   const int64_t it64 = it_done;
