@@ -19,27 +19,38 @@ from .problem import CsrMatrix
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # the current stream's handle without a Stream object around it (a small operator apply
+    # is bound by the host's share of the call)
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _rowmajor(t: torch.Tensor, name: str) -> int:
-    if t.dim() != 2 or t.stride(1) != 1:
+    strides = t.stride()
+    if len(strides) != 2 or strides[1] != 1:
         raise ValueError(f"{name} must be a 2-D row-major tensor")
-    return t.stride(0)
+    return strides[0]
+
+
+def _by_dtype(base: str) -> dict:
+    return {torch.float64: getattr(lib, base + "_f64"), torch.float32: getattr(lib, base + "_f32")}
+
+
+_FNS = {base: _by_dtype(base) for base in ("fe_spmm_csr", "fe_cheb_step", "fe_cheb_filter",
+                                           "fe_gram", "fe_rotate", "fe_residual_norms",
+                                           "fe_column_norms")}
 
 
 def _fn(base: str, t: torch.Tensor):
-    if t.dtype == torch.float64:
-        return getattr(lib, base + "_f64")
-    if t.dtype == torch.float32:
-        return getattr(lib, base + "_f32")
-    raise TypeError(f"unsupported dtype {t.dtype}")
+    fn = _FNS[base].get(t.dtype)
+    if fn is None:
+        raise TypeError(f"unsupported dtype {t.dtype}")
+    return fn
 
 
 def spmm(A: CsrMatrix, X: torch.Tensor, Y: torch.Tensor, alpha: float = 1.0, beta: float = 0.0):
     """Y[:, :b] = alpha*A*X + beta*Y (b = X.shape[1])."""
     ldx, ldy = _rowmajor(X, "X"), _rowmajor(Y, "Y")
-    check(_fn("fe_spmm_csr", X)(A.handle, X.data_ptr(), ldx, Y.data_ptr(), ldy, X.shape[1],
+    check(_fn("fe_spmm_csr", X)(A.handle, X.data_ptr(), ldx, Y.data_ptr(), ldy, X.size(1),
                                 float(alpha), float(beta), _stream()))
     return Y
 
