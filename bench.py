@@ -570,7 +570,7 @@ def measured_peaks():
 def profile_traffic():
     """DRAM bytes per launch of the Chebyshev step from the committed ncu summary
     (scaled to the full workload as that summary states), or None."""
-    p = ROOT / "profiles" / "cheb_step_f32_wells.md"
+    p = ROOT / "profiles" / "cheb_step_f32_wells_rows.md"
     if not p.exists():
         return None
     m = re.search(r"traffic_bytes_per_full_launch:\s*([0-9.eE+]+)", p.read_text())
@@ -599,7 +599,7 @@ def solve_opts(a, precision, seed, locking=None):
     return o
 
 
-SPMM_KERNEL_NAMES = {0: "csr_spmm_row_kernel<float,2,5,7>", 1: "csr_spmm_kernel<float,4,32,*>",
+SPMM_KERNEL_NAMES = {0: "spmm_rows_kernel<float,4,16,1,1,7>", 1: "csr_spmm_kernel<float,4,32,*>",
                      2: "csr_spmm_pipe_kernel<float,4,*>", 3: "csr_spmm_row_kernel<float,4,2,7>",
                      4: "csr_spmm_row_kernel<float,2,5,7> (Z prefetched to L2)",
                      5: "csr_spmm_row_kernel<float,4,3,7>", 6: "csr_spmm_row_kernel<float,2,3,7>",
