@@ -572,32 +572,57 @@ __device__ __forceinline__ void tri_factor(const double* __restrict__ d,
 }
 
 // x <- (T - lambda I)^{-1} x with the factors above (one thread). The running values
-// stay in registers, so each step's chain is one multiply-add and no load waits on a store.
+// stay in registers and the operands of eight steps are read before the first of them, so
+// that a step's chain is one multiply-add and no load waits on a store.
 __device__ __forceinline__ void tri_solve(int k, const double* __restrict__ u0,
                                           const double* __restrict__ u1,
                                           const double* __restrict__ u2,
                                           const double* __restrict__ l,
                                           const double* __restrict__ piv,
                                           double* __restrict__ x) {
+  constexpr int U = 8;
   double xi = x[0];
-#pragma unroll 8
-  for (int i = 0; i + 1 < k; ++i) {
-    const double xn = x[i + 1];
-    const double li = l[i];
-    const bool swap = piv[i] != 0.0;
+  auto forward = [&](double xn, double li, double sw) {
+    const bool swap = sw != 0.0;
     const double a = swap ? xn : xi, b = swap ? xi : xn;
-    x[i] = a;
     xi = fma(-li, a, b);
+    return a;
+  };
+  int i = 0;
+  for (; i + U < k; i += U) {
+    double xn[U], li[U], sw[U];
+#pragma unroll
+    for (int j = 0; j < U; ++j) {
+      xn[j] = x[i + 1 + j];
+      li[j] = l[i + j];
+      sw[j] = piv[i + j];
+    }
+#pragma unroll
+    for (int j = 0; j < U; ++j) x[i + j] = forward(xn[j], li[j], sw[j]);
   }
+  for (; i + 1 < k; ++i) x[i] = forward(x[i + 1], l[i], piv[i]);
   x[k - 1] = xi;
   double x1 = 0.0, x2 = 0.0;  // x[i + 1], x[i + 2]
-#pragma unroll 8
-  for (int i = k - 1; i >= 0; --i) {
-    const double r = fma(-u1[i], x1, fma(-u2[i], x2, x[i] * u0[i]));
-    x[i] = r;
+  auto backward = [&](double b, double c0, double c1, double c2) {
+    const double r = fma(-c1, x1, fma(-c2, x2, b * c0));
     x2 = x1;
     x1 = r;
+    return r;
+  };
+  i = k - 1;
+  for (; i + 1 >= U; i -= U) {
+    double b[U], c0[U], c1[U], c2[U];
+#pragma unroll
+    for (int j = 0; j < U; ++j) {
+      b[j] = x[i - j];
+      c0[j] = u0[i - j];
+      c1[j] = u1[i - j];
+      c2[j] = u2[i - j];
+    }
+#pragma unroll
+    for (int j = 0; j < U; ++j) x[i - j] = backward(b[j], c0[j], c1[j], c2[j]);
   }
+  for (; i >= 0; --i) x[i] = backward(x[i], u0[i], u1[i], u2[i]);
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -605,24 +630,79 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-// One warp per cluster start: eigenvectors of tridiagonal p into Z_T (column-major,
-// ldz) for the cluster's eigenvalues. Scratch: 6 k doubles per eigenvalue index, in shared
-// memory (SMEM; 6 k per warp) or, past its size, in `scratch`. One thread runs the factor
-// and the solves, so the time is the chain of its loads and operations.
-template <bool SMEM>
-__global__ void stein_kernel(const int32_t* __restrict__ msz, const double* __restrict__ d,
-                             const double* __restrict__ e, int64_t vec_stride,
-                             const double* __restrict__ W, int64_t ldw,
-                             const double* __restrict__ tnorm_in, double* __restrict__ Z,
-                             int64_t ldz, double* __restrict__ scratch, int64_t scratch_stride) {
+// x -= (z_q . x) z_q for q = q0 .. q1 - 1 in turn, by one warp, x in shared memory. Up to
+// 32 NE entries stay in registers and the next vector is loaded ahead: a step is then one
+// dot product's shuffles (NE = 0: any length, x and the vectors read again each time).
+template <int NE>
+__device__ __forceinline__ void project_out(const double* __restrict__ Zp, int64_t ldz, int q0,
+                                            int q1, int k, int lane, double* x) {
+  if constexpr (NE == 0) {
+    for (int q = q0; q < q1; ++q) {
+      const double* zq = Zp + static_cast<int64_t>(q) * ldz;
+      double dot = 0.0;
+      for (int i = lane; i < k; i += 32) dot += zq[i] * x[i];
+      dot = warp_sum(dot);
+      for (int i = lane; i < k; i += 32) x[i] -= dot * zq[i];
+      __syncwarp();
+    }
+  } else {
+    if (q0 >= q1) return;
+    double xr[NE], z[NE], zn[NE];
+#pragma unroll
+    for (int e = 0; e < NE; ++e) {
+      const int i = lane + 32 * e;
+      xr[e] = i < k ? x[i] : 0.0;
+      zn[e] = i < k ? Zp[static_cast<int64_t>(q0) * ldz + i] : 0.0;
+    }
+    for (int q = q0; q < q1; ++q) {
+      double dot = 0.0;
+#pragma unroll
+      for (int e = 0; e < NE; ++e) {
+        const int i = lane + 32 * e;
+        z[e] = zn[e];
+        if (q + 1 < q1 && i < k) zn[e] = Zp[static_cast<int64_t>(q + 1) * ldz + i];
+        dot += z[e] * xr[e];
+      }
+      dot = warp_sum(dot);
+#pragma unroll
+      for (int e = 0; e < NE; ++e) xr[e] -= dot * z[e];
+    }
+#pragma unroll
+    for (int e = 0; e < NE; ++e)
+      if (lane + 32 * e < k) x[lane + 32 * e] = xr[e];
+    __syncwarp();
+  }
+}
+
+// Eigenvectors of tridiagonal p into Z_T (column-major, ldz) by inverse iteration: a factor
+// and three rounds of [scale, solve, project out the cluster's earlier vectors, normalize] for
+// each. One thread runs a factor or a solve, so the time is a chain: of one vector, or of a
+// cluster's vectors one after the other. What of a vector does not wait for the one before
+// it is its factor, its first solve and its first projections, and those are done by all four
+// warps of the CTA, a vector each, for a cluster of three vectors or more; the rest runs in
+// order in the first warp. The operations on each vector, and so its bits, are those of one
+// warp alone (which still does clusters of one and two, four at a time). One cluster of all
+// rows, against a warp alone with x and the vectors in memory: 12 rows 153 -> 90 us, 36 1266
+// -> 528, 128 18.0 -> 5.6 ms; 320 rows in a few clusters 184 -> 42 ms; no cluster, 36 rows
+// 18.3 -> 18.2 us, 320 122 -> 107.
+// Scratch: 6 k doubles per warp in shared memory (SMEM) or, past its size, per eigenvalue
+// index in `scratch`, where one warp does a whole cluster.
+template <bool SMEM, int NE>
+__global__ void __launch_bounds__(128)
+stein_kernel(const int32_t* __restrict__ msz, const double* __restrict__ d,
+             const double* __restrict__ e, int64_t vec_stride, const double* __restrict__ W,
+             int64_t ldw, const double* __restrict__ tnorm_in, double* __restrict__ Z,
+             int64_t ldz, double* __restrict__ scratch, int64_t scratch_stride) {
+  constexpr int kWarps = 4;
   const int p = blockIdx.y;
   const int k = msz[p];
-  const int t0 = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+  const int base = blockIdx.x * kWarps;
+  const int warp = threadIdx.x / 32;
   const int lane = threadIdx.x & 31;
-  if (t0 >= k) return;
+  if (base >= k) return;  // the whole CTA
   double* Zp = Z + static_cast<int64_t>(p) * ldz * ldz;
   if (k == 1) {
-    if (lane == 0) Zp[0] = 1.0;
+    if (threadIdx.x == 0) Zp[0] = 1.0;
     return;
   }
   const double* dp = d + p * vec_stride;
@@ -630,47 +710,86 @@ __global__ void stein_kernel(const int32_t* __restrict__ msz, const double* __re
   const double* wp = W + p * ldw;
   const double tnorm = tnorm_in[p];
   const double gap = kClusterTol * tnorm;
-  if (t0 > 0 && wp[t0] - wp[t0 - 1] <= gap) return;  // not the first of its cluster
-  int t1 = t0;
-  while (t1 + 1 < k && wp[t1 + 1] - wp[t1] <= gap) ++t1;
-  extern __shared__ double stein_sh[];
-  double* s = SMEM ? stein_sh + (threadIdx.x / 32) * 6 * k
-                   : scratch + (static_cast<int64_t>(p) * ldz + t0) * scratch_stride;
-  double *u0 = s, *u1 = s + k, *u2 = s + 2 * k, *l = s + 3 * k, *piv = s + 4 * k, *x = s + 5 * k;
   const double tiny = kEps * fmax(tnorm, kTiny);
-  for (int t = t0; t <= t1; ++t) {
-    if (lane == 0) tri_factor(dp, ep, k, wp[t], tiny, u0, u1, u2, l, piv);
+  extern __shared__ double stein_sh[];
+  auto starts = [&](int t) { return t < k && !(t > 0 && wp[t] - wp[t - 1] <= gap); };
+  auto last = [&](int t) {
+    while (t + 1 < k && wp[t + 1] - wp[t] <= gap) ++t;
+    return t;
+  };
+  // factor, start vector and first solve of vector t in scratch s
+  auto begin = [&](double* s, int t) {
+    double* x = s + 5 * k;
+    if (lane == 0) tri_factor(dp, ep, k, wp[t], tiny, s, s + k, s + 2 * k, s + 3 * k, s + 4 * k);
     for (int i = lane; i < k; i += 32) x[i] = hash_uniform(static_cast<uint64_t>(t) + 1, i);
     __syncwarp();
-    for (int it = 0; it < 3; ++it) {
-      // scale to max |x| = 1, solve, orthogonalize against the cluster's earlier
-      // vectors, normalize
-      double mx = 0.0;
-      for (int i = lane; i < k; i += 32) mx = fmax(mx, fabs(x[i]));
-      for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      const double inv = mx > 0.0 ? 1.0 / mx : 1.0;
-      for (int i = lane; i < k; i += 32) x[i] *= inv;
-      __syncwarp();
-      if (lane == 0) tri_solve(k, u0, u1, u2, l, piv, x);
-      __syncwarp();
-      for (int q = t0; q < t; ++q) {
-        const double* zq = Zp + static_cast<int64_t>(q) * ldz;
-        double dot = 0.0;
-        for (int i = lane; i < k; i += 32) dot += zq[i] * x[i];
-        dot = warp_sum(dot);
-        for (int i = lane; i < k; i += 32) x[i] -= dot * zq[i];
-        __syncwarp();
-      }
-      double nn = 0.0;
-      for (int i = lane; i < k; i += 32) nn += x[i] * x[i];
-      nn = warp_sum(nn);
-      const double sc = nn > 0.0 ? 1.0 / sqrt(nn) : 0.0;
-      for (int i = lane; i < k; i += 32) x[i] *= sc;
-      __syncwarp();
+  };
+  // scale to max |x| = 1 and solve
+  auto solve = [&](double* s) {
+    double* x = s + 5 * k;
+    double mx = 0.0;
+    for (int i = lane; i < k; i += 32) mx = fmax(mx, fabs(x[i]));
+    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    const double inv = mx > 0.0 ? 1.0 / mx : 1.0;
+    for (int i = lane; i < k; i += 32) x[i] *= inv;
+    __syncwarp();
+    if (lane == 0) tri_solve(k, s, s + k, s + 2 * k, s + 3 * k, s + 4 * k, x);
+    __syncwarp();
+  };
+  auto normalize = [&](double* x) {
+    double nn = 0.0;
+    for (int i = lane; i < k; i += 32) nn += x[i] * x[i];
+    nn = warp_sum(nn);
+    const double sc = nn > 0.0 ? 1.0 / sqrt(nn) : 0.0;
+    for (int i = lane; i < k; i += 32) x[i] *= sc;
+    __syncwarp();
+  };
+  // the rest of vector t after its first solve and the projections on t0 .. q0 - 1
+  auto finish = [&](double* s, int t0, int q0, int t) {
+    double* x = s + 5 * k;
+    project_out<NE>(Zp, ldz, q0, t, k, lane, x);
+    normalize(x);
+    for (int it = 1; it < 3; ++it) {
+      solve(s);
+      project_out<NE>(Zp, ldz, t0, t, k, lane, x);
+      normalize(x);
     }
     double* zt = Zp + static_cast<int64_t>(t) * ldz;
     for (int i = lane; i < k; i += 32) zt[i] = x[i];
     __syncwarp();
+  };
+
+  if (const int t0 = base + warp; starts(t0)) {
+    double* s = SMEM ? stein_sh + warp * 6 * k
+                     : scratch + (static_cast<int64_t>(p) * ldz + t0) * scratch_stride;
+    const int t1 = last(t0);
+    if (!SMEM || t1 - t0 < 2) {
+      for (int t = t0; t <= t1; ++t) {
+        begin(s, t);
+        solve(s);
+        finish(s, t0, t0, t);
+      }
+    }
+  }
+  if constexpr (SMEM) {
+    for (int t0 = base; t0 < base + kWarps; ++t0) {  // the same for the whole CTA
+      if (!starts(t0)) continue;
+      const int t1 = last(t0);
+      if (t1 - t0 < 2) continue;
+      for (int q = t0; q <= t1; q += kWarps) {
+        __syncthreads();  // the scratch is free; the vectors up to q are written
+        if (const int t = q + warp; t <= t1) {
+          double* s = stein_sh + warp * 6 * k;
+          begin(s, t);
+          solve(s);
+          project_out<NE>(Zp, ldz, t0, q, k, lane, s + 5 * k);
+        }
+        __syncthreads();
+        if (warp == 0)
+          for (int t = q; t <= min(t1, q + kWarps - 1); ++t)
+            finish(stein_sh + (t - q) * 6 * k, t0, q, t);
+      }
+    }
   }
 }
 
@@ -805,7 +924,7 @@ int current_device() {
 // cudaFuncSetAttribute(MaxDynamicSharedMemorySize) once per (kernel slot, device).
 void set_max_smem_once(const void* kernel, int bytes, int dev, int slot) {
   static std::mutex mu;
-  static bool done[5][64] = {};
+  static bool done[7][64] = {};
   std::lock_guard<std::mutex> lock(mu);
   const bool tracked = dev >= 0 && dev < 64;
   if (tracked && done[slot][dev]) return;
@@ -925,15 +1044,18 @@ void syevd_batched_prepared(int count, int kmax, const SyevdWs& w, double* A, in
   FE_CHECK_CUDA(cudaMemsetAsync(Z, 0, sizeof(double) * count * lda * lda, s));
   const size_t stein_smem = size_t(4) * 6 * kmax * sizeof(double);
   const dim3 stein_grid((kmax + 3) / 4, count);
-  if (stein_smem + 1024 <= static_cast<size_t>(optin)) {
-    set_max_smem_once(reinterpret_cast<const void*>(stein_kernel<true>), optin - 256, dev, 3);
-    stein_kernel<true><<<stein_grid, 128, stein_smem, s>>>(w.msz, w.d, w.e, w.vec_stride, W, lda,
-                                                           w.tnorm, Z, lda, w.scratch,
-                                                           w.scratch_stride);
-  } else {
-    stein_kernel<false><<<stein_grid, 128, 0, s>>>(w.msz, w.d, w.e, w.vec_stride, W, lda, w.tnorm,
-                                                   Z, lda, w.scratch, w.scratch_stride);
-  }
+  const bool stein_sh = stein_smem + 1024 <= static_cast<size_t>(optin);
+  auto stein = [&](auto kernel, size_t smem, int slot) {
+    if (smem) set_max_smem_once(reinterpret_cast<const void*>(kernel), optin - 256, dev, slot);
+    kernel<<<stein_grid, 128, smem, s>>>(w.msz, w.d, w.e, w.vec_stride, W, lda, w.tnorm, Z, lda,
+                                         w.scratch, w.scratch_stride);
+  };
+  // A lane's entries of a vector stay in registers up to 12 (128 rows in one cluster: 5.6 ms
+  // against 18.0 in memory); longer vectors are read again for each projection.
+  if (kmax <= 128) stein(stein_kernel<true, 4>, stein_smem, 3);
+  else if (kmax <= 384) stein(stein_kernel<true, 12>, stein_smem, 5);
+  else if (stein_sh) stein(stein_kernel<true, 0>, stein_smem, 6);
+  else stein(stein_kernel<false, 0>, 0, 0);
   check_launch("stein_kernel");
   const size_t orm_smem = ormtr_smem_bytes(kmax);
   if (orm_smem + 1024 <= static_cast<size_t>(optin)) {
