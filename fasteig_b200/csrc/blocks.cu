@@ -97,16 +97,17 @@ gram_partial_kernel(const T* __restrict__ X, int64_t ldx, const T* __restrict__ 
   }
 }
 
-// Sum of the chunks' partials in a fixed order: eight shares of the chunks an output, then
+// Sum of the chunks' partials in a fixed order: SHARES shares of the chunks an output, then
 // the shares in order. With sym_tile > 0 (k == m, only tiles of that side on and above the
-// diagonal computed) an entry below the diagonal tiles reads its mirror (j, i). (One thread
-// per output walking all chunks: 21 us for 48 x 48 and 141 chunks, 4 us so.)
-constexpr int kReduceShares = 8;
-
-__global__ void __launch_bounds__(32 * kReduceShares)
+// diagonal computed) an entry below the diagonal tiles reads its mirror (j, i). The time is
+// the loads' latency where outputs are few, so there a share has hardly more chunks than it
+// loads at once. (One thread per output walking all chunks: 21 us for 48 x 48 and 141 chunks,
+// 4 us in eight shares.)
+template <int SHARES>
+__global__ void __launch_bounds__(32 * SHARES)
 gram_reduce_kernel(const double* __restrict__ partial, int chunks, int k, int m,
                    double* __restrict__ G, int64_t ldg, int sym_tile) {
-  __shared__ double part[kReduceShares][32];
+  __shared__ double part[SHARES][32];
   const int lane = threadIdx.x & 31, share = threadIdx.x >> 5;
   const int64_t idx = static_cast<int64_t>(blockIdx.x) * 32 + lane;
   const int64_t total = static_cast<int64_t>(k) * m;
@@ -116,17 +117,19 @@ gram_reduce_kernel(const double* __restrict__ partial, int chunks, int k, int m,
     const int64_t src =
         (sym_tile && i / sym_tile > j / sym_tile) ? static_cast<int64_t>(i) * k + j : idx;
     double s = 0.0;
-#pragma unroll 4
-    for (int c = share; c < chunks; c += kReduceShares)
+#pragma unroll 8
+    for (int c = share; c < chunks; c += SHARES)
       s += partial[static_cast<int64_t>(c) * total + src];
     part[share][lane] = s;
   }
   __syncthreads();
   if (share == 0 && idx < total) {
-    double s = 0.0;
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-    for (int q = 0; q < kReduceShares; ++q) s += part[q][lane];
-    G[static_cast<int64_t>(j) * ldg + i] = s;
+    for (int q = 0; q < SHARES; q += 4)
+#pragma unroll
+      for (int r = 0; r < 4; ++r) s[r] += part[q + r][lane];
+    G[static_cast<int64_t>(j) * ldg + i] = (s[0] + s[1]) + (s[2] + s[3]);
   }
 }
 
@@ -611,8 +614,16 @@ int launch_gram_partial(const T* X, int64_t ldx, const T* Y, int64_t ldy, int64_
 
 void gram_reduce(const double* partial, const GramPlan& p, int64_t k, int64_t m, double* G,
                  int64_t ldg, int sym_tile, cudaStream_t s) {
-  gram_reduce_kernel<<<static_cast<unsigned>((k * m + 31) / 32), 32 * kReduceShares, 0, s>>>(
-      partial, p.chunks, static_cast<int>(k), static_cast<int>(m), G, ldg, sym_tile);
+  const unsigned grid = static_cast<unsigned>((k * m + 31) / 32);
+  const int ki = static_cast<int>(k), mi = static_cast<int>(m);
+  // 32 shares where one wave of such CTAs holds the output (us, in 8 and in 32: 12 x 12, 216
+  // chunks, 5.8, 4.4; 48 x 48, 296 chunks, 6.9, 3.4; 96 x 96 28.0, 26.9; but 288 x 288, where
+  // the bytes count, 25.5, 35.0)
+  if (p.chunks > 64 && grid <= static_cast<unsigned>(2 * num_sms())) {
+    gram_reduce_kernel<32><<<grid, 32 * 32, 0, s>>>(partial, p.chunks, ki, mi, G, ldg, sym_tile);
+  } else {
+    gram_reduce_kernel<8><<<grid, 32 * 8, 0, s>>>(partial, p.chunks, ki, mi, G, ldg, sym_tile);
+  }
   check_launch("gram_reduce_kernel");
 }
 
