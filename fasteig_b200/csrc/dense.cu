@@ -845,8 +845,7 @@ Csr* csr_create(int64_t rows, int64_t cols, int64_t nnz, const int32_t* rowptr,
   A->nnz = nnz;
   for (int64_t i = 0; i < rows; ++i)
     A->max_row_nnz = std::max<int64_t>(A->max_row_nnz, rowptr[i + 1] - rowptr[i]);
-  const int64_t mid = rows / 2, some = std::min<int64_t>(32, rows - mid);
-  csr_find_grid(*A, rowptr + mid, colind + (rows > 0 ? rowptr[mid] : 0), mid, some);
+  csr_find_grid(*A, rowptr, colind);
   FE_CHECK_CUDA(cudaGetDevice(&A->device));
   try {
     FE_CHECK_CUDA(cudaMalloc(&A->rowptr, (rows + 1) * sizeof(int32_t)));

@@ -9,6 +9,7 @@
 #include <string>
 
 #include "../../include/fasteig_b200.h"
+#include "spmm_grid.hpp"
 
 namespace fe {
 
@@ -103,8 +104,10 @@ struct Csr {
   // multi-step filter (-1: not measured yet)
   mutable int64_t bandwidth = -1;
   // Rows from line to line and from plane to plane of the grid that the diagonals show
-  // (csr_find_grid; 0: none seen). Orders the row blocks of spmm_rows.cu, nothing else.
+  // (csr_find_grid; 0: none seen), and what the rows are like. Chooses and orders the work
+  // of spmm_rows.cu, nothing else.
   int grid_s1 = 0, grid_s2 = 0;
+  RowKind row_kind = RowKind::kUnknown;
   // SpMM kernel chosen by fe_csr_autotune per precision (0 FP64, 1 FP32) for up
   // to four block widths; mode < 0 marks an empty entry.
   struct Tuned {
@@ -116,10 +119,9 @@ struct Csr {
 
 int num_sms();
 
-// The grid behind the operator's diagonals, from a few rows of it on the host (rowptr and
-// colind start at row `row0`) or on the device (spmm_rows.cu).
-void csr_find_grid(Csr& A, const int32_t* rowptr, const int32_t* colind, int64_t row0,
-                   int64_t count);
+// The grid behind the operator's diagonals, from a few rows of it: its arrays on the host, or
+// those on the device (spmm_rows.cu).
+void csr_find_grid(Csr& A, const int32_t* rowptr, const int32_t* colind);
 void csr_find_grid_device(Csr& A);
 // Y = alpha A X + gamma X + beta Z (+ R diag(delta) if R), several rows to a warp
 // (spmm_rows.cu); false, with nothing launched, where it does not apply.

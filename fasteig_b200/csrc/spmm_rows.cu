@@ -384,60 +384,49 @@ void launch(RowsParams<T> P, int64_t rows, bool tail, cudaStream_t s) {
   check_launch("spmm_rows_kernel");
 }
 
-// Line and plane strides of the grid behind a row's column offsets: runs of offsets that
-// differ by 1 are one neighbour along the line (s1: the centre of the first run past the
-// line's own neighbours), runs of those that differ by up to two lines one plane.
-void grid_strides(const int32_t* cols, int count, int64_t row, int64_t rows, int* s1, int* s2) {
-  *s1 = *s2 = 0;
-  std::vector<int> d;
-  for (int i = 0; i < count; ++i)
-    if (cols[i] > row) d.push_back(static_cast<int>(cols[i] - row));
-  std::sort(d.begin(), d.end());
-  size_t i = 0;
-  while (i < d.size() && d[i] < 4) ++i;
-  if (i == d.size()) return;
-  size_t j = i;
-  while (j + 1 < d.size() && d[j + 1] - d[j] <= 1) ++j;
-  const int line = (d[i] + d[j]) / 2;
-  if (line < 4 || line > rows / 2) return;
-  *s1 = line;
-  i = j + 1;
-  while (i < d.size() && d[i] <= 3 * line) ++i;
-  if (i == d.size()) return;
-  j = i;
-  while (j + 1 < d.size() && d[j + 1] - d[j] <= 2 * line + 2) ++j;
-  const int plane = (d[i] + d[j]) / 2;
-  if (plane % line == 0 && plane <= rows / 2) *s2 = plane;
-}
-
 }  // namespace
 
-// Looks at the longest of a few rows in the middle of the operator (a heuristic: the result
-// only orders the work).
-void csr_find_grid(Csr& A, const int32_t* rowptr, const int32_t* colind, int64_t row0,
-                   int64_t count) {
-  A.grid_s1 = A.grid_s2 = 0;
-  int64_t best = -1;
-  for (int64_t i = 0; i < count; ++i)
-    if (best < 0 || rowptr[i + 1] - rowptr[i] > rowptr[best + 1] - rowptr[best]) best = i;
-  if (best < 0) return;
-  grid_strides(colind + (rowptr[best] - rowptr[0]), rowptr[best + 1] - rowptr[best], row0 + best,
-               A.rows, &A.grid_s1, &A.grid_s2);
+// Looks at 32 rows each in the middle and at the quarters of the operator (a heuristic: the
+// result only orders the work).
+constexpr int64_t kGridRows = 32;
+static int64_t grid_window(int64_t rows, int i) {
+  const int64_t quarter[] = {2, 1, 3};
+  return rows / 4 * quarter[i] - kGridRows / 2;
+}
+
+static void set_pattern(Csr& A, const std::vector<RowWindow>& w) {
+  const RowPattern p = find_pattern(w, A.rows);
+  A.grid_s1 = p.s1;
+  A.grid_s2 = p.s2;
+  A.row_kind = p.kind;
+}
+
+void csr_find_grid(Csr& A, const int32_t* rowptr, const int32_t* colind) {
+  std::vector<RowWindow> w;
+  for (int i = 0; i < 3 && A.rows >= 8 * kGridRows; ++i) {
+    const int64_t r = grid_window(A.rows, i);
+    w.push_back({rowptr + r, colind + rowptr[r], r, static_cast<int>(kGridRows)});
+  }
+  set_pattern(A, w);
 }
 
 // The same for an operator whose arrays are on the device.
 void csr_find_grid_device(Csr& A) {
-  A.grid_s1 = A.grid_s2 = 0;
-  if (A.rows < 64 || A.nnz == 0) return;
-  const int64_t row0 = A.rows / 2 - 16, count = 32;
-  std::vector<int32_t> rp(count + 1);
-  FE_CHECK_CUDA(cudaMemcpy(rp.data(), A.rowptr + row0, rp.size() * sizeof(int32_t),
-                           cudaMemcpyDeviceToHost));
-  std::vector<int32_t> ci(std::max(1, rp[count] - rp[0]));
-  if (rp[count] > rp[0])
-    FE_CHECK_CUDA(cudaMemcpy(ci.data(), A.colind + rp[0], (rp[count] - rp[0]) * sizeof(int32_t),
+  std::vector<RowWindow> w;
+  std::vector<int32_t> rp[3], ci[3];
+  for (int i = 0; i < 3 && A.rows >= 8 * kGridRows; ++i) {
+    const int64_t r = grid_window(A.rows, i);
+    rp[i].resize(kGridRows + 1);
+    FE_CHECK_CUDA(cudaMemcpy(rp[i].data(), A.rowptr + r, rp[i].size() * sizeof(int32_t),
                              cudaMemcpyDeviceToHost));
-  csr_find_grid(A, rp.data(), ci.data(), row0, count);
+    const int64_t entries = rp[i][kGridRows] - rp[i][0];
+    ci[i].resize(entries);
+    if (entries > 0)
+      FE_CHECK_CUDA(cudaMemcpy(ci[i].data(), A.colind + rp[i][0], entries * sizeof(int32_t),
+                               cudaMemcpyDeviceToHost));
+    w.push_back({rp[i].data(), ci[i].data(), r, static_cast<int>(kGridRows)});
+  }
+  set_pattern(A, w);
 }
 
 template <typename T>
@@ -500,7 +489,12 @@ bool csr_spmm_rows(const Csr& A, const T* X, int64_t ldx, T* Y, int64_t ldy, con
   //   31, 45);
   // - element-wide lanes: FP32 (113 columns, 57^3: 95, 136); FP64 where the row kernel's lanes
   //   are full (149 columns, 71^3: 334, 356, but 70 columns, 55^3: 140, 88) and, with longer
-  //   rows, up to 224 columns (193, 42^3: 129, 142, but 275, 38^3: 244, 153).
+  //   rows, up to 224 columns (193, 42^3: 129, 142, but 275, 38^3: 244, 153);
+  // - scattered entries (a row's loads come from L2 one by one, and the row kernel has a whole
+  //   short row in flight): rows of more than 48 vectors (200 FP32 columns, 64^3 permuted:
+  //   243, 288), FP32 rows of up to 8 (32 columns, 100^3 permuted: 166, 181), and more than 8
+  //   entries a row (64 FP32 columns, 13 points, 64^3 permuted: 90, 111) but for FP32 columns
+  //   that end inside a vector, which go by elements there (51 columns: 142, 128).
   const int64_t block = A.rows * bytes;
   if (A.rows < 32768) return false;
   if (!tail && (block < (int64_t(16) << 20) || (bytes >= 1024 && block < (int64_t(32) << 20)) ||
@@ -508,6 +502,11 @@ bool csr_spmm_rows(const Csr& A, const T* X, int64_t ldx, T* Y, int64_t ldy, con
     return false;
   if (k > 16 && (bytes > 768 || vec != V16 || bytes <= (tail ? 128 : 256))) return false;
   if (vec == 1 && (sizeof(T) == 4 || (k <= 7 ? ncols < 32 || ncols > 96 : ncols <= 224)))
+    return false;
+  const bool scattered = A.row_kind == RowKind::kScattered;
+  if (scattered &&
+      (bytes > 768 || (k > 8 && (sizeof(T) == 8 || vec != V16 || !tail)) ||
+       (sizeof(T) == 4 && bytes <= 128)))
     return false;
   const int nvec = static_cast<int>((ncols + vec - 1) / vec);
   auto panels = [&](int cap) {
@@ -540,6 +539,7 @@ bool csr_spmm_rows(const Csr& A, const T* X, int64_t ldx, T* Y, int64_t ldy, con
     // 0: (8, 1), 1: (8, 2), 2: (8, 3), 3: (16, 1), 4: (16, 2), 5: (16, 3), 6: (32, 3)
     int shape = 3;
     if (nvec <= 8) shape = 0;
+    else if (scattered && f64) shape = 3;
     else if (nvec <= 16) shape = f64 && k <= 8 ? 3 : 1;
     else if (nvec <= 24) shape = 2;
     else if (nvec <= 32) shape = f64 && k <= 8 ? 3 : 4;
