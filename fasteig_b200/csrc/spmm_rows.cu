@@ -14,8 +14,8 @@
 // plane are read while L1 still holds them: 57 % of the loads hit L1 against 24 % for
 // consecutive rows (128^3, FP32 step of 320 columns: 1.91 ms with one warp per row, 2.35 ms
 // with consecutive rows here, 1.67 ms in bricks, 1.27 ms of DRAM traffic). The brick is
-// only an order: any strides s1 (line) and s2 (plane, a multiple of s1) number every row
-// once.
+// only an order (spmm_grid.hpp): any strides s1 (line) and s2 (plane, a multiple of s1)
+// number every row once.
 //
 // A row's arithmetic is that of the kernel of spmm.cu which such a block would have there,
 // bit for bit: with FOLD, alpha and gamma are folded into the coefficients (the row
@@ -57,10 +57,9 @@ struct RowsParams {
   int ldx, ldy, ldz, ldr;  // bytes from row to row
   int nrows, last_x;       // rows; the last row of X
   int ncols, pc, panels;   // columns of the block and of a panel, panels
-  int lbx;                 // log2 of a brick's rows along a line
-  int s1, s2;              // rows from line to line, from plane to plane
-  int lines;               // lines of a plane
-  int nx, ny, bz;          // bricks along a line and across a plane, planes of a brick
+  int s1, s2, lines;       // order of the rows (RowOrder)
+  int lbx, nx, ny;
+  int bz;                  // planes that a brick sweeps down
   T alpha, gamma, beta;
   int use_gamma, use_beta;
 };
@@ -87,10 +86,7 @@ spmm_rows_kernel(const __grid_constant__ RowsParams<T> P) {
   const int grp = threadIdx.x / G;
   const int panel = blockIdx.x % P.panels;  // panels side by side: whole rows from DRAM
   const int brick = blockIdx.x / P.panels;
-  const int bx = brick % P.nx, byz = brick / P.nx;
-  const int by = byz % P.ny, bz = byz / P.ny;
-  const int x = (bx << P.lbx) + (grp & ((1 << P.lbx) - 1));
-  const int y = by * (NG >> P.lbx) + (grp >> P.lbx);
+  const RowPlace at0 = row_place(brick, grp, P.lbx, NG >> P.lbx, P.nx, P.ny);
   const int c0 = panel * P.pc;
   const int nvec = (min(P.pc, P.ncols - c0) + VEC - 1) / VEC;
   bool act[CPL];
@@ -121,8 +117,9 @@ spmm_rows_kernel(const __grid_constant__ RowsParams<T> P) {
     return p + static_cast<int64_t>(row) * pitch;
   };
   const unsigned mine = G == 32 ? kFull : ((1u << (G & 31)) - 1u) << (lane - gl);
-  const bool in = x < P.s1 && y < P.lines;
-  int64_t r64 = x + static_cast<int64_t>(P.s1) * y + static_cast<int64_t>(P.s2) * bz * P.bz;
+  const bool in = at0.x < P.s1 && at0.y < P.lines;
+  const int64_t r64 = at0.x + static_cast<int64_t>(P.s1) * at0.y +
+                      static_cast<int64_t>(P.s2) * at0.z * P.bz;
   int row = in && r64 < P.nrows ? static_cast<int>(r64) : -1;
   int zi = 0;
   auto next_of = [&](int r) {
@@ -349,22 +346,13 @@ spmm_rows_kernel(const __grid_constant__ RowsParams<T> P) {
 template <typename T, int VEC, int G, int CPL, int M, int KC, bool FOLD, bool CORR>
 void launch(RowsParams<T> P, int64_t rows, bool tail, cudaStream_t s) {
   constexpr int NG = kRowsThreads / G;
-  // Bricks of 4 lines; without a grid the "planes" are runs of NG consecutive rows.
-  int by = NG / 4;
-  if (P.s1 == 0) {
-    P.s1 = P.s2 = NG;
-    P.lines = 1;
-    by = 1;
-  } else if (P.s2 == 0) {  // a grid of lines only: sweep down groups of `by` lines
-    P.lines = by;
-    P.s2 = P.s1 * by;
-  } else {
-    P.lines = P.s2 / P.s1;
-  }
-  P.lbx = 0;
-  while ((by << P.lbx) < NG) ++P.lbx;
-  P.nx = (P.s1 + (1 << P.lbx) - 1) >> P.lbx;
-  P.ny = (P.lines + by - 1) / by;
+  const RowOrder order = row_order(P.s1, P.s2, NG);
+  P.s1 = order.s1;
+  P.s2 = order.s2;
+  P.lines = order.lines;
+  P.lbx = order.lbx;
+  P.nx = order.nx;
+  P.ny = order.ny;
   const int64_t planes = (rows + P.s2 - 1) / P.s2;
   const int64_t columns = static_cast<int64_t>(P.nx) * P.ny * P.panels;
   // A CTA's first rows wait for a chain of loads that the later ones hide, and deep bricks
@@ -438,12 +426,9 @@ bool csr_spmm_rows(const Csr& A, const T* X, int64_t ldx, T* Y, int64_t ldy, con
   const int k = static_cast<int>(std::min<int64_t>(A.max_row_nnz, 64));
   const int64_t bytes = ncols * static_cast<int64_t>(sizeof(T));
   const int64_t far = std::max(std::max(ldx, ldy), std::max(ub ? ldz : 0, R ? ldr : 0));
-  // A vector's columns fit the wide row kernel better than panels without a grid's reuse:
-  // 320 FP32 columns take 1.91 ms there and 2.35 ms here (128^3); 160 columns 714 against
-  // 475 us (96^3). Blocks of up to four vectors keep the loop kernel's smaller groups.
+  // Blocks of up to four vectors keep the loop kernel's smaller groups.
   if (k < 1 || k > 32 || bytes <= 64 || far * static_cast<int64_t>(sizeof(T)) > 0x7fffffffLL)
     return false;
-  if (A.grid_s1 == 0 && bytes > 1024) return false;
   auto multiple = [&](size_t b) {
     auto ok = [b](const void* p, int64_t ld) {
       return reinterpret_cast<uintptr_t>(p) % b == 0 && (ld * sizeof(T)) % b == 0;
@@ -490,25 +475,41 @@ bool csr_spmm_rows(const Csr& A, const T* X, int64_t ldx, T* Y, int64_t ldy, con
   // - element-wide lanes: FP32 (113 columns, 57^3: 95, 136); FP64 where the row kernel's lanes
   //   are full (149 columns, 71^3: 334, 356, but 70 columns, 55^3: 140, 88) and, with longer
   //   rows, up to 224 columns (193, 42^3: 129, 142, but 275, 38^3: 244, 153);
+  // - rows of more than 64 vectors that do not fill panels of 32, in blocks of up to 64 MB
+  //   (320 FP32 columns, 35^3: 43, 48) and on grids of small planes (5 x 80 x 800: 284, 305),
+  //   and any row of more than 64 vectors on thinner grids, short lines with far couplings and
+  //   operators of unknown rows (10 x 10 x 4000: 355, 355; lines of 77 rows and a coupling
+  //   100,003 rows off: 262, 283; but 600 x 600, 297, 242, and tridiagonal, 234, 189);
   // - scattered entries (a row's loads come from L2 one by one, and the row kernel has a whole
   //   short row in flight): rows of more than 48 vectors (200 FP32 columns, 64^3 permuted:
   //   243, 288), FP32 rows of up to 8 (32 columns, 100^3 permuted: 166, 181), and more than 8
   //   entries a row (64 FP32 columns, 13 points, 64^3 permuted: 90, 111) but for FP32 columns
   //   that end inside a vector, which go by elements there (51 columns: 142, 128).
-  const int64_t block = A.rows * bytes;
+  const int64_t block = A.rows * bytes, MB = int64_t(1) << 20;
+  const int nvec = static_cast<int>((ncols + vec - 1) / vec);
+  const int lanes16 = (nvec + 15) / 16 * 16, lanes32 = (nvec + 31) / 32 * 32;
+  const bool panels32 = lanes32 * 19 <= lanes16 * 20;
   if (A.rows < 32768) return false;
-  if (!tail && (block < (int64_t(16) << 20) || (bytes >= 1024 && block < (int64_t(32) << 20)) ||
-                (bytes <= 128 && block < (int64_t(64) << 20))))
+  if (!tail && (block < 16 * MB || (bytes >= 1024 && block < 32 * MB) ||
+                (bytes <= 192 && block < 24 * MB) || (bytes <= 128 && block < 64 * MB)))
     return false;
   if (k > 16 && (bytes > 768 || vec != V16 || bytes <= (tail ? 128 : 256))) return false;
   if (vec == 1 && (sizeof(T) == 4 || (k <= 7 ? ncols < 32 || ncols > 96 : ncols <= 224)))
     return false;
+  const Sweep sweep = row_sweep(A.grid_s1, A.grid_s2);
   const bool scattered = A.row_kind == RowKind::kScattered;
+  if (bytes > 1024) {
+    if (sweep == Sweep::kRuns && A.row_kind != RowKind::kBanded &&
+        A.row_kind != RowKind::kIrregular && (k <= 8 || A.row_kind != RowKind::kGrid))
+      return false;
+    if (k <= 8 && !panels32 &&
+        (block < 64 * MB || (sweep == Sweep::kPlanes && A.grid_s2 < kSmallPlane)))
+      return false;
+  }
   if (scattered &&
       (bytes > 768 || (k > 8 && (sizeof(T) == 8 || vec != V16 || !tail)) ||
        (sizeof(T) == 4 && bytes <= 128)))
     return false;
-  const int nvec = static_cast<int>((ncols + vec - 1) / vec);
   auto panels = [&](int cap) {
     P.panels = (nvec + cap - 1) / cap;
     P.pc = (nvec + P.panels - 1) / P.panels * vec;
@@ -532,20 +533,26 @@ bool csr_spmm_rows(const Csr& A, const T* X, int64_t ldx, T* Y, int64_t ldy, con
     // columns 194 (16, 3) against 220). Wider rows: panels of (16, 2) where they fill their
     // lanes (256 columns 544 against 574), else of (16, 1) with a whole short row in flight
     // (320 columns, 128^3: 1.67 against 1.80 ms). FP64 rows of 9 to 16 and 25 to 32 vectors
-    // do as well or better in (16, 1) panels.
-    const int lanes16 = (nvec + 15) / 16 * 16, lanes32 = (nvec + 31) / 32 * 32;
+    // do as well or better in (16, 1) panels where a sweep is deep or, with irregular rows, L1
+    // has little to give; elsewhere (8, 2) and (16, 2) (us: 24 columns of a 600 x 600 grid 98
+    // -> 66, 64 columns of a 40000 x 8 grid 133 -> 111), and (8, 2) for the widest (320 FP32
+    // columns, 600 x 600: 430 -> 242).
     const int lanes24 = (nvec + 23) / 24 * 24;
     const bool f64 = sizeof(T) == 8;
+    const bool deep = sweep == Sweep::kPlanes ? A.rows / 16 >= A.grid_s2
+                                              : A.row_kind != RowKind::kGrid &&
+                                                    A.row_kind != RowKind::kBanded;
     // 0: (8, 1), 1: (8, 2), 2: (8, 3), 3: (16, 1), 4: (16, 2), 5: (16, 3), 6: (32, 3)
     int shape = 3;
     if (nvec <= 8) shape = 0;
     else if (scattered && f64) shape = 3;
-    else if (nvec <= 16) shape = f64 && k <= 8 ? 3 : 1;
+    else if (nvec <= 16) shape = f64 && k <= 8 && deep ? 3 : 1;
     else if (nvec <= 24) shape = 2;
-    else if (nvec <= 32) shape = f64 && k <= 8 ? 3 : 4;
+    else if (nvec <= 32) shape = f64 && k <= 8 && deep ? 3 : 4;
     else if (nvec <= 48) shape = 5;
     else if (k > 8 && k <= 16 && nvec > 64 && nvec <= 96) shape = 6;
-    else if (lanes32 * 19 <= lanes16 * 20) shape = f64 && k <= 8 ? 3 : 4;
+    else if (panels32) shape = f64 && k <= 8 && deep ? 3 : 4;
+    else if (k <= 8 && !deep) shape = 1;
     else if (lanes24 < lanes16) shape = 2;
     if (k > 16 && shape < 3) shape = nvec <= 16 ? 3 : 4;  // 8 lanes hold 16 entries
 #define FE_SHAPES(CORR_)                                          \

@@ -1,6 +1,8 @@
-"""What the multi-row SpMM takes an operator's rows to be (fasteig_b200/csrc/spmm_grid.hpp,
-compiled with g++ through tests/cpp/grid_check.cpp): the strides found on grids, and none on
-scattered, permuted or banded operators."""
+"""The order in which the multi-row SpMM deals rows to its groups of lanes
+(fasteig_b200/csrc/spmm_grid.hpp, compiled with g++ through tests/cpp/grid_check.cpp): every
+row once and none outside its plane, also at sizes where an int product of two strides would
+overflow; groups kept busy on thin grids and far couplings; the strides found on grids, and
+none on scattered, permuted or banded operators."""
 import shutil
 import subprocess
 from pathlib import Path
@@ -27,6 +29,31 @@ def exe(tmp_path_factory):
 def run(exe, what, text):
     r = subprocess.run([str(exe), what], input=text, capture_output=True, text=True, check=True)
     return [float(v) for v in r.stdout.split()]
+
+
+# rows, line, plane: cubes, thin and flat grids, far couplings, lines only, no grid
+ORDERS = [(117649, 49, 2401), (262144, 64, 4096), (40000, 10, 100), (32771, 4, 16),
+          (60000, 5, 1025), (60000, 7, 1400), (90000, 300, 30000), (66000, 1023, 2046),
+          (60000, 20000, 0), (60000, 30000, 0), (90000, 300, 0), (70000, 130, 0),
+          (70000, 2047, 0), (70000, 77, 0), (33333, 0, 0)]
+
+
+@pytest.mark.parametrize("groups", [8, 16, 32])
+@pytest.mark.parametrize("rows,s1,s2", ORDERS)
+def test_every_row_once_and_groups_busy(exe, rows, s1, s2, groups):
+    wrong, outside, used = run(exe, "deal", f"{rows} {s1} {s2} {groups}")
+    assert wrong == 0 and outside == 0
+    assert used >= 0.75
+
+
+@pytest.mark.parametrize("s1,s2", [(268435455, 0), (1073741823, 0), (16384, 268435456),
+                                   (5, 268435455), (536870911, 1073741822), (0, 0)])
+@pytest.mark.parametrize("groups", [8, 16, 32])
+def test_order_at_the_index_limit(exe, s1, s2, groups):
+    o1, o2, lines, bx, bricks, last = run(exe, "place", f"2147483646 {s1} {s2} {groups}")
+    assert o1 * lines == o2 <= 2 ** 30
+    assert bricks * groups >= o2 and bricks < 2 ** 31
+    assert last == o2 - 1  # the last brick ends with the plane's last row
 
 
 UNKNOWN, GRID, BANDED, IRREGULAR, SCATTERED = range(5)

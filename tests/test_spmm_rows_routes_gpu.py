@@ -1,6 +1,7 @@
-"""The multi-row SpMM on operators without a grid: bands with and without repeating offsets,
-permuted rows; FP64 rows at odd pitches with folded coefficients; and the correction term of
-the refined filter through whole solves.
+"""The multi-row SpMM on every kind of operator that its dispatch tells apart: planes (also
+thin ones), lines (short, long, couplings as far as half the rows), bands with and without
+repeating offsets, permuted rows; FP64 rows at odd pitches with folded coefficients; and the
+correction term of the refined filter through whole solves.
 References: the product in 64 bits from SciPy, with the bound of test_spmm_rows_gpu.py (an
 output is a chain of at most 15 rounded multiply-adds: 32 units of the type's rounding of the
 sum of the terms' sizes), and, bit for bit, the kernels of one warp per row (mode 7), whose
@@ -53,6 +54,16 @@ def _operator(kind):
         return _csr(n, rows, cols, 1)
     return {
         "tridiagonal": lambda: _diagonals(n, (-1, 0, 1), 2),
+        "half": lambda: _diagonals(n, (-(n // 2), -1, 0, 1, n // 2), 3),
+        "third": lambda: _diagonals(39999, (-13333, -1, 0, 1, 13333), 4),
+        "far": lambda: _diagonals(n, (-15013, -77, 0, 77, 15013), 5),
+        "thin": lambda: _grid((10, 10, 401), "star1", 6),
+        "thin16": lambda: _grid((16, 16, 150), "star1", 7),
+        "sliver": lambda: _grid((5, 90, 80), "star1", 8),
+        "flat": lambda: _grid((120, 115, 3), "star1", 9),
+        "lines": lambda: _grid((197, 201), "star1", 10),
+        "long_lines": lambda: _grid((2100, 19), "star1", 11),
+        "thin13": lambda: _grid((9, 9, 500), "star2", 12),
         "permuted": lambda: _grid((34, 34, 35), "star1", 13, permute=True),
         "permuted13": lambda: _grid((34, 34, 35), "star2", 14, permute=True),
     }[kind]()
@@ -93,7 +104,9 @@ def _check(H, cols, ld, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
-@pytest.mark.parametrize("kind", ["tridiagonal", "band", "permuted", "permuted13"])
+@pytest.mark.parametrize("kind", ["tridiagonal", "band", "half", "third", "far", "thin", "thin16",
+                                  "sliver", "flat", "lines", "long_lines", "thin13", "permuted",
+                                  "permuted13"])
 @pytest.mark.parametrize("cols,ld", [(51, 56), (64, 64), (109, 112), (128, 128), (322, 328),
                                      (512, 512)])
 def test_kinds_of_operators(kind, cols, ld, dtype):
