@@ -303,21 +303,23 @@ __global__ void bks_end_kernel(BatchLayout L, BatchState S) {
 // the 2 x 2 blocks (pair, pair) of A through both sides of the rotation in registers, so A
 // goes through shared memory once a round, not twice, and a round has two barriers; the
 // next round's rotations (a chain of divisions and roots) are formed beside Q's update;
-// blocks and Q's elements are dealt to 1024 threads once, before the sweeps (a call of 8
-// matrices of 96: 4.76 ms with one side after the other on 256 threads, 1.80 ms so, the
-// same results bit for bit).
-constexpr int kJacThreads = 1024;
+// blocks and Q's elements are dealt to the threads once, before the sweeps (a call of 8
+// matrices of 96: 4.76 ms with one side after the other on 256 threads, 1.80 ms so on 1024,
+// the same results bit for bit: no sum depends on the number of threads).
 constexpr int kJacMaxHalf = kBatchMaxDim / 2;
-constexpr int kJacBlocks = (kJacMaxHalf * kJacMaxHalf + kJacThreads - 1) / kJacThreads;
-constexpr int kJacRotThreads = 64;  // form the next round's rotations beside Q's update
-constexpr int kJacQThreads = kJacThreads - kJacRotThreads;
-constexpr int kJacQ = (kJacMaxHalf * kBatchMaxDim + kJacQThreads - 1) / kJacQThreads;
-static_assert(kJacMaxHalf <= kJacRotThreads, "a thread per rotation");
+constexpr int kJacSums = 256;  // partial sums of a sweep's check, whatever the threads
 
-__global__ void __launch_bounds__(kJacThreads)
+// THREADS for matrices of up to 2 HALF rows.
+template <int THREADS, int HALF>
+__global__ void __launch_bounds__(THREADS)
 bks_jacobi_kernel(BatchLayout L, const double* __restrict__ T, const int32_t* __restrict__ mdim,
                   int same, const int32_t* __restrict__ todo, double* __restrict__ W,
                   double* __restrict__ Z, double* __restrict__ Zlast) {
+  constexpr int kRot = (HALF + 31) / 32 * 32;  // threads that form the next round's rotations
+  constexpr int kQThreads = THREADS - kRot;    // beside the others' update of Q
+  constexpr int kBlocks = (HALF * HALF + THREADS - 1) / THREADS;
+  constexpr int kQ = (2 * HALF * HALF + kQThreads - 1) / kQThreads;
+  static_assert(kQThreads >= 32 && THREADS % 32 == 0, "a warp for Q beside the rotations");
   extern __shared__ double sh[];
   const int p = blockIdx.x;
   if (todo && !todo[p]) return;
@@ -328,12 +330,12 @@ bks_jacobi_kernel(BatchLayout L, const double* __restrict__ T, const int32_t* __
   double2* rot = reinterpret_cast<double2*>(
       (reinterpret_cast<uintptr_t>(Q + m * ld) + 15) & ~uintptr_t(15));  // (c, s) of a pair, two rounds
   int2* pq = reinterpret_cast<int2*>(rot + 2 * kJacMaxHalf);             // its rows
-  __shared__ double red[2][kJacThreads / 32];
+  __shared__ double red[2][kJacSums / 32];
   __shared__ int done;
   const int tid = threadIdx.x;
   const int64_t M = L.M;
   const double* Tp = T + p * M * M;
-  for (int e = tid; e < m * m; e += kJacThreads) {
+  for (int e = tid; e < m * m; e += THREADS) {
     const int i = e % m, j = e / m;
     A[i + j * ld] = Tp[i + j * M];
     Q[i + j * ld] = i == j ? 1.0 : 0.0;
@@ -341,16 +343,16 @@ bks_jacobi_kernel(BatchLayout L, const double* __restrict__ T, const int32_t* __
   __syncthreads();
   const int mm = m + (m & 1), half = mm / 2;
   // this thread's blocks (k1 | k2 << 16) and elements of Q (pair | row << 16), -1: none
-  int blk[kJacBlocks], qel[kJacQ];
+  int blk[kBlocks], qel[kQ];
 #pragma unroll
-  for (int u = 0; u < kJacBlocks; ++u) {
-    const int e = tid + u * kJacThreads;
+  for (int u = 0; u < kBlocks; ++u) {
+    const int e = tid + u * THREADS;
     blk[u] = e < half * half ? (e / half) | ((e % half) << 16) : -1;
   }
 #pragma unroll
-  for (int u = 0; u < kJacQ; ++u) {
-    const int e = tid - kJacRotThreads + u * kJacQThreads;
-    qel[u] = tid >= kJacRotThreads && e < half * m ? (e / m) | ((e % m) << 16) : -1;
+  for (int u = 0; u < kQ; ++u) {
+    const int e = tid - kRot + u * kQThreads;
+    qel[u] = tid >= kRot && e < half * m ? (e / m) | ((e % m) << 16) : -1;
   }
   auto rotations = [&](int round) {  // pair tid of the round
     const int k = tid;
@@ -380,25 +382,27 @@ bks_jacobi_kernel(BatchLayout L, const double* __restrict__ T, const int32_t* __
     pq[at] = make_int2(lo, hi < m ? hi : lo);
   };
   for (int sweep = 0; sweep < 40; ++sweep) {
-    double off = 0.0, dg = 0.0;
-    for (int e = tid; e < m * m; e += kJacThreads) {
-      const int i = e % m, j = e / m;
-      const double a = A[i + j * ld];
-      if (i == j) dg = fma(a, a, dg);
-      else off = fma(a, a, off);
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      off += __shfl_xor_sync(0xffffffffu, off, o);
-      dg += __shfl_xor_sync(0xffffffffu, dg, o);
-    }
-    if (tid % 32 == 0) {
-      red[0][tid / 32] = off;
-      red[1][tid / 32] = dg;
+    for (int t = tid; t < kJacSums; t += THREADS) {  // whole warps
+      double off = 0.0, dg = 0.0;
+      for (int e = t; e < m * m; e += kJacSums) {
+        const int i = e % m, j = e / m;
+        const double a = A[i + j * ld];
+        if (i == j) dg = fma(a, a, dg);
+        else off = fma(a, a, off);
+      }
+      for (int o = 16; o > 0; o >>= 1) {
+        off += __shfl_xor_sync(0xffffffffu, off, o);
+        dg += __shfl_xor_sync(0xffffffffu, dg, o);
+      }
+      if (t % 32 == 0) {
+        red[0][t / 32] = off;
+        red[1][t / 32] = dg;
+      }
     }
     __syncthreads();
     if (tid == 0) {
       double off_s = 0.0, dg_s = 0.0;
-      for (int w = 0; w < kJacThreads / 32; ++w) {
+      for (int w = 0; w < kJacSums / 32; ++w) {
         off_s += red[0][w];
         dg_s += red[1][w];
       }
@@ -413,7 +417,7 @@ bks_jacobi_kernel(BatchLayout L, const double* __restrict__ T, const int32_t* __
       const int2* rp = pq + (round & 1) * kJacMaxHalf;
       // A <- J^T (A J), block by block
 #pragma unroll
-      for (int u = 0; u < kJacBlocks; ++u) {
+      for (int u = 0; u < kBlocks; ++u) {
         if (blk[u] < 0) continue;
         const int k1 = blk[u] & 0xffff, k2 = blk[u] >> 16;
         const double2 r1 = rr[k1], r2 = rr[k2];
@@ -446,7 +450,7 @@ bks_jacobi_kernel(BatchLayout L, const double* __restrict__ T, const int32_t* __
       // Q <- Q J, and the next round's rotations from the new A
       if (tid < half && round + 1 < mm - 1) rotations(round + 1);
 #pragma unroll
-      for (int u = 0; u < kJacQ; ++u) {
+      for (int u = 0; u < kQ; ++u) {
         if (qel[u] < 0) continue;
         const int k = qel[u] & 0xffff, i = qel[u] >> 16;
         const double2 r = rr[k];
@@ -462,7 +466,7 @@ bks_jacobi_kernel(BatchLayout L, const double* __restrict__ T, const int32_t* __
   // Ascending order (stable by index on ties), as a rank per diagonal entry.
   int* place = reinterpret_cast<int*>(rot);
   __syncthreads();
-  for (int i = tid; i < m; i += kJacThreads) {
+  for (int i = tid; i < m; i += THREADS) {
     const double di = A[i + i * ld];
     int rank = 0;
     for (int j = 0; j < m; ++j) {
@@ -474,7 +478,7 @@ bks_jacobi_kernel(BatchLayout L, const double* __restrict__ T, const int32_t* __
     place[i] = rank;
   }
   __syncthreads();
-  for (int e = tid; e < m * m; e += kJacThreads) {
+  for (int e = tid; e < m * m; e += THREADS) {
     const int r = e % m, i = e / m;
     Z[p * M * M + r + static_cast<int64_t>(place[i]) * M] = Q[r + i * ld];
   }
@@ -693,10 +697,26 @@ size_t bks_jacobi_smem(int m) {
 void bks_jacobi(const BatchLayout& L, const double* T, const int32_t* mdim, const int32_t* todo,
                 int max_m, double* W, double* Z, double* Zlast, cudaStream_t s, int same) {
   const size_t smem = bks_jacobi_smem(max_m);
-  FE_CHECK_CUDA(cudaFuncSetAttribute(bks_jacobi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(smem)));
-  bks_jacobi_kernel<<<static_cast<unsigned>(L.num_problems), kJacThreads, smem, s>>>(
-      L, T, mdim, same, todo, W, Z, Zlast);
+  auto run = [&](auto kernel, int threads) {
+    FE_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       static_cast<int>(smem)));
+    kernel<<<static_cast<unsigned>(L.num_problems), threads, smem, s>>>(L, T, mdim, same, todo, W,
+                                                                        Z, Zlast);
+  };
+  // us for that many matrices, with (128, 256) threads up to 32 rows, (256, 768) up to 64:
+  //            148        512         3000
+  //   8 rows   51, 48     51, 50      119, 163
+  //   20       128, 110   145, 137    543, 657
+  //   48       522, 399   1086, 1540  5588, 7878
+  //   64       1102, 793  2731, 2774  12262, 14462
+  // (1024 threads for every size: 51, 137, 630; 114, 400, 1991; 418, 1616, 8266; 796, 2789,
+  // 14545). So: the threads that make one matrix quickest while a CTA has its SM to itself,
+  // fewer where several share it.
+  if (max_m > 64) run(bks_jacobi_kernel<1024, kJacMaxHalf>, 1024);
+  else if (max_m > 32 && L.num_problems <= num_sms()) run(bks_jacobi_kernel<768, 32>, 768);
+  else if (max_m > 32) run(bks_jacobi_kernel<256, 32>, 256);
+  else if (L.num_problems <= 4 * num_sms()) run(bks_jacobi_kernel<256, 16>, 256);
+  else run(bks_jacobi_kernel<128, 16>, 128);
   check_launch("bks_jacobi_kernel");
 }
 
