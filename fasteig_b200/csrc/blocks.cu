@@ -245,11 +245,11 @@ rotate_kernel(const T* __restrict__ X, int64_t ldx, const double* __restrict__ C
 // Three streams (AX, M X, R) at two rounded operations a value: DRAM bound. One CTA per SM
 // takes a run of whole rows; its threads are dealt over the row's 16-byte vectors and over
 // rows, four rows of a thread in flight, so that every row is read in full lines and the
-// SM has up to 190 KB under way. (One warp per 32 columns, a value a lane and a row at a
+// SM has 128 KB of loads under way. (One warp per 32 columns, a value a lane and a row at a
 // time, took 477 us a call for 512,000 x 96 FP64 with B and R, 2.5 TB/s; this takes 223 us,
 // 5.3 TB/s.)
 constexpr int kNormThreads = 1024;
-constexpr int kNormMaxVecs = 512;  // vectors of a row that one CTA takes
+constexpr int kNormMaxVecs = 512;  // vectors of a row that one CTA takes at most
 constexpr int kNormMaxChunks = 148;
 constexpr int kNormRows = 4;  // rows of a thread in flight
 
@@ -266,11 +266,11 @@ __global__ void __launch_bounds__(kNormThreads)
 residual_partial_kernel(const T* __restrict__ AX, const T* __restrict__ X,
                         const T* __restrict__ BX, int64_t ld, int64_t n, int m,
                         const double* __restrict__ lambda, T* __restrict__ R, int64_t ldr,
-                        int64_t rows_per_chunk, double* __restrict__ partial) {
+                        int64_t rows_per_chunk, int block_cols, double* __restrict__ partial) {
   using V = NormVec<T, VEC>;
   extern __shared__ double red[];  // [row share][2][columns of this CTA]
-  const int col0 = blockIdx.x * kNormMaxVecs * VEC;
-  const int cols = min(m - col0, kNormMaxVecs * VEC);
+  const int col0 = blockIdx.x * block_cols;
+  const int cols = min(m - col0, block_cols);
   const int vecs = cols / VEC;  // exact: VEC > 1 only where VEC divides m
   const int shares = kNormThreads / vecs;
   const int share = threadIdx.x / vecs;
@@ -368,15 +368,35 @@ __global__ void residual_finish_kernel(const double* __restrict__ partial, int c
 }
 
 struct NormPlan {
-  int chunks;
+  int blocks, block_cols, chunks;
   int64_t rows_per_chunk;
   size_t bytes;
 };
 
-// Row chunks: one CTA per SM, of 64 rows at least.
-NormPlan norm_plan(int64_t n, int64_t m) {
+// Rows of a chunk at least: 64, or fewer where rows are so wide that only a few share a CTA's
+// threads, which then take them one after the other (50 rows of 2048 FP32 columns, residual:
+// 39 us in one chunk, 17 in seven).
+int64_t norm_min_rows(int64_t m) {
+  return std::max<int64_t>(8, std::min<int64_t>(64, 8192 / std::max<int64_t>(m, 1)));
+}
+
+// Column blocks of at most kNormMaxVecs vectors of VEC values, and row chunks: one CTA per SM
+// over both. One block more than the columns need where that keeps the threads much busier
+// (350 vectors: 700 of 1024 in one block, 875 in two).
+NormPlan norm_plan(int64_t n, int64_t m, int vec) {
   NormPlan p{};
-  const int64_t chunks = std::max<int64_t>(1, std::min<int64_t>(kNormMaxChunks, (n + 63) / 64));
+  const int64_t vecs = std::max<int64_t>(1, m / vec);
+  auto used = [&](int64_t blocks) {
+    const int64_t v = (vecs + blocks - 1) / blocks;
+    return kNormThreads / v * v;
+  };
+  int64_t blocks = (vecs + kNormMaxVecs - 1) / kNormMaxVecs;
+  if (used(blocks) < kNormThreads * 3 / 4 && used(blocks + 1) > used(blocks)) ++blocks;
+  p.block_cols = static_cast<int>((vecs + blocks - 1) / blocks * vec);
+  p.blocks = static_cast<int>((m + p.block_cols - 1) / p.block_cols);
+  const int64_t least = norm_min_rows(m);
+  const int64_t most = std::max<int64_t>(1, kNormMaxChunks / std::max(1, p.blocks));
+  const int64_t chunks = std::max<int64_t>(1, std::min<int64_t>(most, (n + least - 1) / least));
   p.rows_per_chunk = std::max<int64_t>(1, (n + chunks - 1) / chunks);
   p.chunks = static_cast<int>(std::max<int64_t>(1, (n + p.rows_per_chunk - 1) / p.rows_per_chunk));
   p.bytes = static_cast<size_t>(p.chunks) * 2 * std::max<int64_t>(m, 1) * sizeof(double);
@@ -392,9 +412,8 @@ void launch_residual(const T* AX, const T* X, const T* BX, int64_t ld, int64_t n
   const size_t smem = static_cast<size_t>(2) * kNormThreads * VEC * sizeof(double);
   FE_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      static_cast<int>(smem)));
-  const int blocks = (m + kNormMaxVecs * VEC - 1) / (kNormMaxVecs * VEC);
-  kern<<<dim3(blocks, p.chunks), kNormThreads, smem, s>>>(AX, X, BX, ld, n, m, lambda, R, ldr,
-                                                          p.rows_per_chunk, partial);
+  kern<<<dim3(p.blocks, p.chunks), kNormThreads, smem, s>>>(
+      AX, X, BX, ld, n, m, lambda, R, ldr, p.rows_per_chunk, p.block_cols, partial);
   check_launch("residual_partial_kernel");
 }
 
@@ -744,10 +763,11 @@ template void rotate<float>(const float*, int64_t, const double*, int64_t, float
                             int64_t, int64_t, int64_t, double, double, cudaStream_t, bool);
 
 // Bound valid for every call with n' <= n and m' <= m (chunks never exceed the
-// target count nor one per 64 rows).
+// target count nor one per norm_min_rows(m) rows, which narrower blocks only raise).
 size_t residual_workspace_bytes(int64_t n, int64_t m) {
   if (n <= 0 || m <= 0) return 0;
-  const int64_t chunks = std::min<int64_t>(256, (n + 63) / 64 + 1);
+  const int64_t least = norm_min_rows(m);
+  const int64_t chunks = std::min<int64_t>(256, (n + least - 1) / least + 1);
   return static_cast<size_t>(chunks) * 2 * m * sizeof(double);
 }
 
@@ -763,18 +783,20 @@ void residual_norms(const T* AX, const T* X, const T* BX, int64_t ld, int64_t n,
   if (mode == 2) FE_REQUIRE(BX, "residual_norms: B-norms need BX");
   if (R) FE_REQUIRE(ldr >= m, "residual_norms: invalid R leading dimension");
   FE_REQUIRE(m <= 65535LL * 32, "residual_norms: too many columns");
-  const NormPlan p = norm_plan(std::max<int64_t>(n, 1), m);
+  constexpr int V16 = 16 / sizeof(T);
+  auto rows16 = [](const T* q, int64_t pitch) { return !q || (aligned16(q) && pitch % V16 == 0); };
+  const int vec = m % V16 == 0 && rows16(AX, ld) && rows16(X, ld) && rows16(BX, ld) &&
+                          rows16(R, ldr)
+                      ? V16
+                      : 1;
+  const NormPlan p = norm_plan(std::max<int64_t>(n, 1), m, vec);
   FE_REQUIRE(ws && ws_bytes >= p.bytes, "residual_norms: workspace too small");
   if (n == 0) {
     FE_CHECK_CUDA(cudaMemsetAsync(ws, 0, p.bytes, s));
   } else {
-    constexpr int V16 = 16 / sizeof(T);
-    auto rows16 = [](const T* q, int64_t pitch) { return !q || (aligned16(q) && pitch % V16 == 0); };
-    const bool vec = m % V16 == 0 && rows16(AX, ld) && rows16(X, ld) && rows16(BX, ld) &&
-                     rows16(R, ldr);
     double* partial = static_cast<double*>(ws);
     const int cols = static_cast<int>(m);
-    if (vec)
+    if (vec == V16)
       launch_residual<T, V16>(AX, X, BX, ld, n, cols, lambda, R, ldr, p, partial, mode, s);
     else
       launch_residual<T, 1>(AX, X, BX, ld, n, cols, lambda, R, ldr, p, partial, mode, s);
