@@ -243,15 +243,17 @@ rotate_kernel(const T* __restrict__ X, int64_t ldx, const double* __restrict__ C
 
 // -------------------------------------------------- Residual and norms ----
 // Three streams (AX, M X, R) at two rounded operations a value: DRAM bound. One CTA per SM
-// takes a run of whole rows; its threads are dealt over the row's 16-byte vectors and over
-// rows, four rows of a thread in flight, so that every row is read in full lines and the
-// SM has 128 KB of loads under way. (One warp per 32 columns, a value a lane and a row at a
-// time, took 477 us a call for 512,000 x 96 FP64 with B and R, 2.5 TB/s; this takes 223 us,
-// 5.3 TB/s.)
+// takes a run of whole rows; its threads are dealt over the row's vectors (16 bytes where the
+// rows allow it) and over rows, two to sixteen rows of a thread in flight, so that every row
+// is read in full lines and the SM has 64 KB of loads under way. (One warp per 32
+// columns, a value a lane and a row at a time, took 477 us a call for 512,000 x 96 FP64 with B
+// and R, 2.5 TB/s; this takes 223 us, 5.3 TB/s.)
 constexpr int kNormThreads = 1024;
 constexpr int kNormMaxVecs = 512;  // vectors of a row that one CTA takes at most
 constexpr int kNormMaxChunks = 148;
-constexpr int kNormRows = 4;  // rows of a thread in flight
+// Rows of a thread in flight: 64 bytes of one stream, 32 of each of two (with 64 of each the FP32
+// residual spills: 500,000 rows of 256 columns 418 us so, 245 us with 32).
+constexpr int norm_rows(int vec_bytes, int mode) { return (mode == 0 ? 64 : 32) / vec_bytes; }
 
 template <typename T, int VEC>
 struct __align__(VEC * sizeof(T)) NormVec {
@@ -268,6 +270,7 @@ residual_partial_kernel(const T* __restrict__ AX, const T* __restrict__ X,
                         const double* __restrict__ lambda, T* __restrict__ R, int64_t ldr,
                         int64_t rows_per_chunk, int block_cols, double* __restrict__ partial) {
   using V = NormVec<T, VEC>;
+  constexpr int kRows = norm_rows(VEC * static_cast<int>(sizeof(T)), MODE);
   extern __shared__ double red[];  // [row share][2][columns of this CTA]
   const int col0 = blockIdx.x * block_cols;
   const int cols = min(m - col0, block_cols);
@@ -285,10 +288,29 @@ residual_partial_kernel(const T* __restrict__ AX, const T* __restrict__ X,
   }
   if (share < shares) {
     const T* M = BX ? BX : X;
-    for (int64_t r0 = r_begin + share; r0 < r_end; r0 += kNormRows * shares) {
-      V mx[kNormRows], ax[kNormRows];
+    int64_t r0 = r_begin + share;
+    if constexpr (MODE == 0 && VEC * sizeof(T) < 16) {
+      // narrow vectors of one stream: whole batches of rows without a check (500,000 rows,
+      // norms, us: 51 FP32 columns 64 -> 29, 201 226 -> 89, 201 FP64 212 -> 144)
+      const T* p = M + r0 * ld + j;
+      const int64_t step = static_cast<int64_t>(shares) * ld;
+      for (; r0 + (kRows - 1) * shares < r_end; r0 += kRows * shares, p += kRows * step) {
+        V v[kRows];
 #pragma unroll
-      for (int u = 0; u < kNormRows; ++u) {
+        for (int u = 0; u < kRows; ++u) v[u] = *reinterpret_cast<const V*>(p + u * step);
+#pragma unroll
+        for (int u = 0; u < kRows; ++u)
+#pragma unroll
+          for (int e = 0; e < VEC; ++e) {
+            const double x = static_cast<double>(v[u].v[e]);
+            sx[e] = fma(x, x, sx[e]);
+          }
+      }
+    }
+    for (; r0 < r_end; r0 += kRows * shares) {
+      V mx[kRows], ax[kRows];
+#pragma unroll
+      for (int u = 0; u < kRows; ++u) {
         const int64_t r = r0 + u * shares;
         if (r < r_end) {
           mx[u] = *reinterpret_cast<const V*>(M + r * ld + j);
@@ -297,7 +319,7 @@ residual_partial_kernel(const T* __restrict__ AX, const T* __restrict__ X,
         }
       }
 #pragma unroll
-      for (int u = 0; u < kNormRows; ++u) {
+      for (int u = 0; u < kRows; ++u) {
         const int64_t r = r0 + u * shares;
         if (r < r_end) {
           V out;
@@ -783,12 +805,15 @@ void residual_norms(const T* AX, const T* X, const T* BX, int64_t ld, int64_t n,
   if (mode == 2) FE_REQUIRE(BX, "residual_norms: B-norms need BX");
   if (R) FE_REQUIRE(ldr >= m, "residual_norms: invalid R leading dimension");
   FE_REQUIRE(m <= 65535LL * 32, "residual_norms: too many columns");
+  // whole vectors of 16 bytes, or of 8 in FP32, where the rows are made of them
+  auto made_of = [&](int v) {
+    auto ok = [v](const T* q, int64_t pitch) {
+      return !q || (reinterpret_cast<uintptr_t>(q) % (v * sizeof(T)) == 0 && pitch % v == 0);
+    };
+    return m % v == 0 && ok(AX, ld) && ok(X, ld) && ok(BX, ld) && ok(R, ldr);
+  };
   constexpr int V16 = 16 / sizeof(T);
-  auto rows16 = [](const T* q, int64_t pitch) { return !q || (aligned16(q) && pitch % V16 == 0); };
-  const int vec = m % V16 == 0 && rows16(AX, ld) && rows16(X, ld) && rows16(BX, ld) &&
-                          rows16(R, ldr)
-                      ? V16
-                      : 1;
+  const int vec = made_of(V16) ? V16 : sizeof(T) == 4 && m >= 32 && made_of(2) ? 2 : 1;
   const NormPlan p = norm_plan(std::max<int64_t>(n, 1), m, vec);
   FE_REQUIRE(ws && ws_bytes >= p.bytes, "residual_norms: workspace too small");
   if (n == 0) {
@@ -798,6 +823,8 @@ void residual_norms(const T* AX, const T* X, const T* BX, int64_t ld, int64_t n,
     const int cols = static_cast<int>(m);
     if (vec == V16)
       launch_residual<T, V16>(AX, X, BX, ld, n, cols, lambda, R, ldr, p, partial, mode, s);
+    else if (sizeof(T) == 4 && vec == 2)
+      launch_residual<T, 2>(AX, X, BX, ld, n, cols, lambda, R, ldr, p, partial, mode, s);
     else
       launch_residual<T, 1>(AX, X, BX, ld, n, cols, lambda, R, ldr, p, partial, mode, s);
   }
