@@ -308,9 +308,10 @@ int gram_dmma_tile(int64_t k, int64_t m, bool symmetric) {
   for (int t = 0; t < 3; ++t) {
     const double tk = static_cast<double>((k + kTiles[t] - 1) / kTiles[t]);
     const double tm = static_cast<double>((m + kTiles[t] - 1) / kTiles[t]);
+    if (tm > 65535 && kTiles[t] < 64) continue;  // the launch's limit
     const double tiles = symmetric ? tk * (tk + 1) / 2 : tk * tm;
     const double cost = tiles * kTiles[t] * kTiles[t] / kRate[t];
-    if (t == 0 || cost < least) {
+    if (least == 0.0 || cost < least) {
       least = cost;
       best = kTiles[t];
     }
@@ -329,6 +330,7 @@ int rotate_tile(int64_t k, int64_t m, bool upper_tri) {
   int best = 32;
   int64_t least = -1;
   for (int t : kTiles) {
+    if (least >= 0 && (m + t - 1) / t > 65535) continue;  // the launch's limit
     int64_t cost = 0;
     for (int64_t j = 0; j < m; j += t) cost += t * (upper_tri ? std::min<int64_t>(k, j + t) : k);
     if (least < 0 || cost < least) {
