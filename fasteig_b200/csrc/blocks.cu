@@ -133,6 +133,23 @@ gram_reduce_kernel(const double* __restrict__ partial, int chunks, int k, int m,
   }
 }
 
+// The same for a few chunks, a thread per output.
+__global__ void __launch_bounds__(256)
+gram_sum_kernel(const double* __restrict__ partial, int chunks, int k, int m,
+                double* __restrict__ G, int64_t ldg, int sym_tile) {
+  const int64_t idx = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x;
+  const int64_t total = static_cast<int64_t>(k) * m;
+  if (idx >= total) return;
+  const int i = static_cast<int>(idx % k);
+  const int j = static_cast<int>(idx / k);
+  const int64_t src =
+      (sym_tile && i / sym_tile > j / sym_tile) ? static_cast<int64_t>(i) * k + j : idx;
+  double s = 0.0;
+#pragma unroll 8
+  for (int c = 0; c < chunks; ++c) s += partial[static_cast<int64_t>(c) * total + src];
+  G[static_cast<int64_t>(j) * ldg + i] = s;
+}
+
 struct GramPlan {
   int tile, tiles_k, tiles_m, chunks;
   int64_t rows_per_chunk;
@@ -662,6 +679,8 @@ void gram_reduce(const double* partial, const GramPlan& p, int64_t k, int64_t m,
   // the bytes count, 25.5, 35.0)
   if (p.chunks > 64 && grid <= static_cast<unsigned>(2 * num_sms())) {
     gram_reduce_kernel<32><<<grid, 32 * 32, 0, s>>>(partial, p.chunks, ki, mi, G, ldg, sym_tile);
+  } else if (p.chunks <= 16) {  // hardly more loads than a thread has in flight
+    gram_sum_kernel<<<(grid + 7) / 8, 256, 0, s>>>(partial, p.chunks, ki, mi, G, ldg, sym_tile);
   } else {
     gram_reduce_kernel<8><<<grid, 32 * 8, 0, s>>>(partial, p.chunks, ki, mi, G, ldg, sym_tile);
   }
