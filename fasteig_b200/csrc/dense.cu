@@ -403,10 +403,35 @@ trinv_upper_block_kernel(const double* __restrict__ R, int64_t ldr, double* __re
     }
     __syncthreads();
   }
+  bool odd = false;
   for (int c = warp; c < cb; c += kTrinvThreads / 32) {
     const int col = J * 32 + c;
-    for (int r = lane; r < k; r += 32)
-      Rinv[static_cast<int64_t>(col) * ldi + r] = r <= col ? X[r * kTrinvLd + c] : 0.0;
+    for (int r = lane; r < k; r += 32) {
+      const double x = r <= col ? X[r * kTrinvLd + c] : 0.0;
+      odd |= !isfinite(x);
+      Rinv[static_cast<int64_t>(col) * ldi + r] = x;
+    }
+  }
+  // A column of the inverse depends on R's columns up to its own, but in the products above a
+  // zero pivot's or another non-finite entry meets the zeros of X below the diagonal in the
+  // columns before it. Then each column again, by back substitution alone.
+  if (!__syncthreads_or(odd)) return;
+  for (int c = warp; c < cb; c += kTrinvThreads / 32) {
+    const int col = J * 32 + c;
+    double* x = X + c;
+    if (lane == 0) x[col * kTrinvLd] = 1.0 / R[static_cast<int64_t>(col) * ldr + col];
+    __syncwarp();
+    for (int i = col - 1; i >= 0; --i) {
+      double sum = 0.0;
+      for (int l = i + 1 + lane; l <= col; l += 32)
+        sum = fma(R[static_cast<int64_t>(l) * ldr + i], x[l * kTrinvLd], sum);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      if (lane == 0) x[i * kTrinvLd] = -sum / R[static_cast<int64_t>(i) * ldr + i];
+      __syncwarp();
+    }
+    for (int r = lane; r <= col; r += 32)
+      Rinv[static_cast<int64_t>(col) * ldi + r] = x[r * kTrinvLd];
   }
 }
 
