@@ -280,6 +280,7 @@ potrf_upper_kernel(double* G, int k, int64_t ldg, int32_t* info, int64_t batch_s
       int bad = 0;
 #pragma unroll
       for (int j = 0; j < 32; ++j) {
+        if (j >= jb) break;  // the padding's pivots are 1
         const double d = __shfl_sync(0xffffffffu, a[j], j);
         if (bad == 0 && (!(d > 0.0) || !isfinite(d))) bad = j + 1;
         const double root = sqrt(d), inv = 1.0 / root;
