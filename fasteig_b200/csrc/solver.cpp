@@ -1644,7 +1644,7 @@ void check_pair(const Csr& A, const Csr& B) {
 // weighted Cholesky QR, src/core/Orthogonalization.cpp:407-440), corrections
 // W = T R with T = diag(|K_ii|)^-1, and the relative residual of
 // evaluate_ritz_pairs with B (src/core/RitzExtraction.cpp:50-56). B absent means
-// M = I (B-blocks are then copies).
+// M = I (the B blocks are then the blocks themselves).
 // ===========================================================================
 template <typename T>
 struct GenBlockOpsT {
@@ -1657,6 +1657,9 @@ struct GenBlockOpsT {
   int64_t n, ld;
   Stats& st;
   DeviceBuffer idx_dev;
+  // Sources of ortho's uploads, one set a pass: they outlive the next wait for the stream.
+  std::vector<int32_t> sel[2] = {};
+  std::vector<double> inv[2] = {};
   // Singular values of an orthonormalization below this fraction of the largest
   // are dropped as noise: about sqrt(unit roundoff) of the block's precision.
   static constexpr double kRankFloor = sizeof(T) == 4 ? 1e-3 : 1e-7;
@@ -1691,7 +1694,7 @@ struct GenBlockOpsT {
     if (k >= n || cols <= 0) return 0;
     const T* cur = src;
     int64_t rank = 0;
-    std::vector<double> norms, w, inv;
+    std::vector<double> norms, w;
     for (int pass = 0; pass < 2; ++pass) {
       bapply(cur, tmpB, cols);
       residual_norms<T>(nullptr, cur, B ? tmpB : cur, ld, n, cols, nullptr, nullptr, 0, nullptr,
@@ -1724,22 +1727,24 @@ struct GenBlockOpsT {
       const double smax = std::sqrt(std::max(w[cols - 1], 0.0));
       const int64_t capacity = std::min<int64_t>(cols, n - k);
       const double cut = std::max(rank_tol * scale, kRankFloor * smax);
-      std::vector<int32_t> sel;
-      inv.clear();
-      for (int64_t i = cols - 1; i >= 0 && static_cast<int64_t>(sel.size()) < capacity; --i) {
+      std::vector<int32_t>& at = sel[pass];
+      std::vector<double>& by = inv[pass];
+      at.clear();
+      by.clear();
+      for (int64_t i = cols - 1; i >= 0 && static_cast<int64_t>(at.size()) < capacity; --i) {
         const double sv = std::sqrt(std::max(w[i], 0.0));
         if (!(sv > cut)) break;
-        sel.push_back(static_cast<int32_t>(i));
-        inv.push_back(1.0 / sv);
+        at.push_back(static_cast<int32_t>(i));
+        by.push_back(1.0 / sv);
       }
-      rank = static_cast<int64_t>(sel.size());
+      rank = static_cast<int64_t>(at.size());
       if (rank == 0) return 0;
       const size_t dbl_off = ((rank * sizeof(int32_t) + 7) / 8) * 8;
       idx_dev.resize(dbl_off + rank * sizeof(double));
       int32_t* di = idx_dev.as<int32_t>();
       double* ds = reinterpret_cast<double*>(idx_dev.as<uint8_t>() + dbl_off);
-      ctx.to_device(di, sel.data(), rank);
-      ctx.to_device(ds, inv.data(), rank);
+      ctx.to_device(di, at.data(), rank);
+      ctx.to_device(ds, by.data(), rank);
       small_gather_scale(G, sm.cap, cols, di, ds, rank, sm.Rinv.as<double>(), sm.cap, s);
       rotate_block<T>(sm, tmp, ld, sm.Rinv.as<double>(), out, ld, n, cols, rank, 1.0, 0.0, s);
       if (B)
