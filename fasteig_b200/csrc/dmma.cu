@@ -89,7 +89,7 @@ gram_dmma_kernel(const double* __restrict__ X, int64_t ldx, const double* __rest
   auto xs = [&](int buf) { return smem + static_cast<size_t>(buf) * 2 * kGR * kGLd; };
   auto ys = [&](int buf) { return xs(buf) + kGR * kGLd; };
 
-  // 16 rows x 64 columns per operand: 1024 / VEC copies over 128 threads.
+  // 16 rows x T columns per operand: 16 T / VEC copies over 128 threads.
   auto load = [&](int t, int buf) {
     const int64_t rb = r_begin + static_cast<int64_t>(t) * kGR;
     double* xd = xs(buf);
@@ -215,7 +215,7 @@ rotate_dmma_kernel(const double* __restrict__ X, int64_t ldx, const double* __re
       const bool in = r < n && kb + kk < k;
       cp_async<8 * VEC>(xd + rr * kRXLd + kk, in ? X + r * ldx + kb + kk : X, in);
     }
-    // C (column-major): 16 inner x 64 columns, one double per copy (the smem
+    // C (column-major): 16 inner x TC columns, one double per copy (the smem
     // tile is transposed relative to the source).
 #pragma unroll
     for (int e = 0; e < (kRK * kRCols) / kRThreads; ++e) {

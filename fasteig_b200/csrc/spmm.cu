@@ -1140,17 +1140,14 @@ int read_spmm_status(bool clear) {
   return v;
 }
 
-// Kernel selection for csr_spmm: "pipe" (bulk-copy pipelined) or "warp" (registers only).
-// 0 = row-batched kernel (panels <= 96 vectors) where it applies, 1 = loop kernel,
-// 2 = bulk-copy pipeline where it applies, 3 = row-batched with panels <= 64 vectors,
-// 4 = mode 0 with the next Z row prefetched into L2.
+// Kernel selection for csr_spmm (csr_spmm_mode; fe_set_spmm_kernel names the modes).
 static int g_spmm_mode = 0;
 void set_spmm_mode(int mode) { g_spmm_mode = mode; }
 
 template <typename T>
 void fill_uniform(T* X, int64_t ld, int64_t n, int64_t m, uint64_t seed, cudaStream_t s);
 
-// Kernel choice for a call: an explicit process-wide mode (1..3) wins; under the
+// Kernel choice for a call: an explicit process-wide mode (1..7) wins; under the
 // default mode a width tuned on this operator by fe_csr_autotune (within a factor
 // of two of ncols) picks the kernel.
 std::mutex g_tune_mutex;
@@ -1208,9 +1205,9 @@ void csr_spmm_mode(int mode, const Csr& A, const T* X, int64_t ldx, T* Y, int64_
   const bool vec_ok = ncols % VEC == 0 && ldx % VEC == 0 && ldy % VEC == 0 && aligned16(X) &&
                       aligned16(Y) && (!ub || (ldz % VEC == 0 && aligned16(Z)));
   if (vec_ok) {
-    // Mode 0: the row-batched register kernel for slabs of >= 32 vectors and rows
-    // of <= 8 nonzeros; mode 2: the bulk-copy pipelined kernel (needs 16-byte
-    // aligned row gathers and rows that fit its stages).
+    // Mode 0 where csr_spmm_rows declined: the row-batched register kernel for slabs of
+    // >= 32 vectors and rows of <= 7 nonzeros; mode 2: the bulk-copy pipelined kernel
+    // (needs 16-byte aligned row gathers and rows that fit its stages).
     // Mode 0 gives each lane 8-byte vectors (up to 5 per lane, so a 320-column
     // FP32 slab needs no idle lanes and ~70 registers of loads in flight); mode 3
     // uses 16-byte vectors with at most 2 per lane.
@@ -1222,7 +1219,7 @@ void csr_spmm_mode(int mode, const Csr& A, const T* X, int64_t ldx, T* Y, int64_
         try_row_kernel<T, VEC>(A, vals, X, ldx, Y, ldy, Z, ldz, static_cast<int>(ncols), T(alpha),
                                T(gamma), T(beta), ug, ub, s, 2))
       return;
-    // Mode 4: mode 0 with the next row's Z row prefetched into L2.
+    // Mode 4: the same kernel with the next row's Z row prefetched into L2.
     if (mode == 4 &&
         try_row_kernel<T, 8 / sizeof(T)>(A, vals, X, ldx, Y, ldy, Z, ldz, static_cast<int>(ncols),
                                          T(alpha), T(gamma), T(beta), ug, ub, s, 5, true))
@@ -1238,7 +1235,7 @@ void csr_spmm_mode(int mode, const Csr& A, const T* X, int64_t ldx, T* Y, int64_
         try_row_kernel<T, 8 / sizeof(T)>(A, vals, X, ldx, Y, ldy, Z, ldz, static_cast<int>(ncols),
                                          T(alpha), T(gamma), T(beta), ug, ub, s, 3))
       return;
-    // Mode 7: mode 0 with X and Z read through L2 only.
+    // Mode 7: the same kernel with X and Z read through L2 only.
     if (mode == 7 &&
         try_row_kernel<T, 8 / sizeof(T)>(A, vals, X, ldx, Y, ldy, Z, ldz, static_cast<int>(ncols),
                                          T(alpha), T(gamma), T(beta), ug, ub, s, 5, false, true))
@@ -1341,8 +1338,8 @@ template void csr_spmm<float>(const Csr&, const float*, int64_t, float*, int64_t
 
 // Y = alpha A X + gamma X + beta Z + R diag(delta) on FP32 blocks: the Chebyshev step
 // of the refined filter's correction recurrence (see refined_filter in the solver).
-// The row-batched kernel carries the extra term in its store; where that kernel does
-// not apply, the step is followed by a separate column-scaled add.
+// The multi-row and the row-batched kernel carry the extra term in their store; where
+// neither applies, the step is followed by a separate column-scaled add.
 void csr_spmm_corr_f32(const Csr& A, const float* X, int64_t ldx, float* Y, int64_t ldy,
                        const float* Z, int64_t ldz, const float* R, int64_t ldr,
                        const float* delta, int64_t ncols, double alpha, double gamma, double beta,

@@ -363,8 +363,9 @@ void launch(RowsParams<T> P, int64_t rows, bool tail, cudaStream_t s) {
   P.bz = std::max(1, std::min(16, static_cast<int>(std::sqrt(share) + 0.5)));
   const int64_t grid = columns * ((planes + P.bz - 1) / P.bz);
   FE_REQUIRE(grid <= 0x7fffffffLL, "csr_spmm: too many rows for one launch");
-  if (VEC > 1 && tail)
-    spmm_rows_kernel<T, VEC, G, CPL, M, KC, FOLD, (VEC > 1), CORR>
+  // a correction comes with whole vectors only
+  if (VEC > 1 && !CORR && tail)
+    spmm_rows_kernel<T, VEC, G, CPL, M, KC, FOLD, (VEC > 1 && !CORR), CORR>
         <<<static_cast<unsigned>(grid), kRowsThreads, 0, s>>>(P);
   else
     spmm_rows_kernel<T, VEC, G, CPL, M, KC, FOLD, false, CORR>
@@ -558,7 +559,7 @@ bool csr_spmm_rows(const Csr& A, const T* X, int64_t ldx, T* Y, int64_t ldy, con
 #define FE_SHAPES(CORR_)                                          \
   do {                                                            \
     if (k <= 8) {                                                 \
-      if (shape == 0) FE_ROWS(V16, 8, 1, 1, 7, CORR_);            \
+      if (shape == 0) FE_ROWS_F(V16, 8, 1, 1, 7, false, CORR_);   \
       if (shape == 1) FE_ROWS(V16, 8, 2, 1, 2, CORR_);            \
       if (shape == 2) FE_ROWS(V16, 8, 3, 1, 2, CORR_);            \
       if (shape == 3) FE_ROWS(V16, 16, 1, 1, 7, CORR_);           \

@@ -201,15 +201,18 @@ int fe_device_status(int32_t* status, int32_t clear);
  * inject_wait_timeout=<code> runs the same probe on a solve's word (test hook). */
 int fe_selftest_wait_timeout(int64_t limit_cycles, int32_t code, void* stream);
 /* SpMM kernel selection for all later calls in the process (the numerics are
- * the same; the choice only changes the memory schedule): 0 = default
- * (several rows to a warp for rows of <= 32 nonzeros, in bricks of the operator's
- * grid; without a grid and with more than 1 KiB of a row the row-batched register
- * kernel for rows of <= 7 nonzeros; else the loop kernel), 1 = loop kernel, 2 = bulk-copy
- * pipelined kernel where it applies, 3 = row-batched kernel with narrower
- * column panels, 4 = mode 0 with each warp's next Z row prefetched into L2,
- * 5 = row-batched kernel with 16-byte lanes and up to 3 per lane, 6 = row-batched
- * kernel with 8-byte lanes and up to 3 per lane, 7 = mode 0 with X and Z read
- * through L2 only (ld.global.cg). */
+ * the same; the choice only changes the memory schedule): 0 = default: several
+ * rows to a warp, in an order taken from the operator's grid, for operators of
+ * 32,768 rows and more with rows of <= 32 nonzeros, where the block's width, size
+ * and alignment and the operator's pattern make that the faster one (the rule, with
+ * times for both sides, is in csr_spmm_rows); otherwise one warp per row with the
+ * row's nonzeros in registers (rows of <= 7 nonzeros, 32 or more 8-byte vectors),
+ * else the loop kernel. 1 = loop kernel, 2 = bulk-copy pipelined kernel where it
+ * applies. The others are variants of the kernel of one warp per row, where it
+ * applies: 3 = 16-byte lanes, at most 2 per lane, 4 = 8-byte lanes with each warp's
+ * next Z row prefetched into L2, 5 = 16-byte lanes and up to 3 per lane, 6 = 8-byte
+ * lanes and up to 3 per lane, 7 = 8-byte lanes with X and Z read through L2 only
+ * (ld.global.cg). */
 int fe_set_spmm_kernel(int32_t mode);
 /* Chebyshev filter schedule for all later filters in the process (fe_cheb_filter_*
  * and the Chebyshev solver; the numerics are the same bit for bit): 0 = default,
