@@ -698,8 +698,9 @@ void bks_jacobi(const BatchLayout& L, const double* T, const int32_t* mdim, cons
                 int max_m, double* W, double* Z, double* Zlast, cudaStream_t s, int same) {
   const size_t smem = bks_jacobi_smem(max_m);
   auto run = [&](auto kernel, int threads) {
+    // the same limit in every call: another thread's smaller batch must not lower it
     FE_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(smem)));
+                                       static_cast<int>(bks_jacobi_smem(kBatchMaxDim))));
     kernel<<<static_cast<unsigned>(L.num_problems), threads, smem, s>>>(L, T, mdim, same, todo, W,
                                                                         Z, Zlast);
   };
