@@ -475,8 +475,11 @@ bool csr_spmm_rows(const Csr& A, const T* X, int64_t ldx, T* Y, int64_t ldy, con
   //   31, 45);
   // - element-wide lanes: FP32 (113 columns, 57^3: 95, 136); FP64 where the row kernel's lanes
   //   are full (149 columns, 71^3: 334, 356, but 70 columns, 55^3: 140, 88) and, with longer
-  //   rows, up to 224 columns (193, 42^3: 129, 142, but 275, 38^3: 244, 153);
-  // - rows of more than 64 vectors that do not fill panels of 32, in blocks of up to 64 MB
+  //   rows, up to 224 columns (193, 42^3: 129, 142, but 275, 38^3: 244, 153), and the 49 to 64
+  //   columns that go in two panels here (51, 64^3: 154, 158; 45, 154, 91; 65, 211, 163);
+  // - FP32 rows of 8-byte lanes, up to 7 entries, where the row kernel's panels (of up to 160
+  //   vectors) take four or five vectors a lane (258 columns, 64^3: 228, 309; 162, 212, 192);
+  // - rows of more than 64 16-byte vectors that do not fill panels of 32, in blocks of up to 64 MB
   //   (320 FP32 columns, 35^3: 43, 48) and on grids of small planes (5 x 80 x 800: 284, 305),
   //   and any row of more than 64 vectors on thinner grids, short lines with far couplings and
   //   operators of unknown rows (10 x 10 x 4000: 355, 355; lines of 77 rows and a coupling
@@ -485,7 +488,9 @@ bool csr_spmm_rows(const Csr& A, const T* X, int64_t ldx, T* Y, int64_t ldy, con
   //   short row in flight): rows of more than 48 vectors (200 FP32 columns, 64^3 permuted:
   //   243, 288), FP32 rows of up to 8 (32 columns, 100^3 permuted: 166, 181), and more than 8
   //   entries a row (64 FP32 columns, 13 points, 64^3 permuted: 90, 111) but for FP32 columns
-  //   that end inside a vector, which go by elements there (51 columns: 142, 128).
+  //   that end inside a vector, which go by elements there (51 columns: 142, 128); 8-byte
+  //   vectors from 33 on with up to 8 entries (98 FP32 columns, 64^3 permuted: 145, 176) and
+  //   FP64 rows by elements from 49 columns on (65: 223, 237).
   const int64_t block = A.rows * bytes, MB = int64_t(1) << 20;
   const int nvec = static_cast<int>((ncols + vec - 1) / vec);
   const int lanes16 = (nvec + 15) / 16 * 16, lanes32 = (nvec + 31) / 32 * 32;
@@ -495,11 +500,17 @@ bool csr_spmm_rows(const Csr& A, const T* X, int64_t ldx, T* Y, int64_t ldy, con
                 (bytes <= 192 && block < 24 * MB) || (bytes <= 128 && block < 64 * MB)))
     return false;
   if (k > 16 && (bytes > 768 || vec != V16 || bytes <= (tail ? 128 : 256))) return false;
-  if (vec == 1 && (sizeof(T) == 4 || (k <= 7 ? ncols < 32 || ncols > 96 : ncols <= 224)))
+  if (vec == 1 &&
+      (sizeof(T) == 4 ||
+       (k <= 7 ? ncols < 32 || (ncols > 48 && ncols <= 64) || ncols > 96 : ncols <= 224)))
     return false;
+  if (sizeof(T) == 4 && vec == 2 && k <= 7) {  // the row kernel's panels of up to 160 vectors
+    const int parts = (nvec + 159) / 160;
+    if ((nvec + parts - 1) / parts > 96) return false;
+  }
   const Sweep sweep = row_sweep(A.grid_s1, A.grid_s2);
   const bool scattered = A.row_kind == RowKind::kScattered;
-  if (bytes > 1024) {
+  if (bytes > 1024 && vec == V16) {
     if (sweep == Sweep::kRuns && A.row_kind != RowKind::kBanded &&
         A.row_kind != RowKind::kIrregular && (k <= 8 || A.row_kind != RowKind::kGrid))
       return false;
@@ -507,10 +518,11 @@ bool csr_spmm_rows(const Csr& A, const T* X, int64_t ldx, T* Y, int64_t ldy, con
         (block < 64 * MB || (sweep == Sweep::kPlanes && A.grid_s2 < kSmallPlane)))
       return false;
   }
-  if (scattered &&
-      (bytes > 768 || (k > 8 && (sizeof(T) == 8 || vec != V16 || !tail)) ||
-       (sizeof(T) == 4 && bytes <= 128)))
-    return false;
+  if (scattered) {
+    const bool whole = vec == V16 && bytes <= 768 && (k <= 8 || (sizeof(T) == 4 && tail));
+    const bool narrow = vec != V16 && (k > 8 || nvec <= (sizeof(T) == 4 ? 32 : 48));
+    if ((!whole && !narrow) || (sizeof(T) == 4 && bytes <= 128)) return false;
+  }
   auto panels = [&](int cap) {
     P.panels = (nvec + cap - 1) / cap;
     P.pc = (nvec + P.panels - 1) / P.panels * vec;

@@ -119,6 +119,16 @@ def test_f64_odd_pitch_folded(cols, ld):
     _check(M.laplacian_wells(37, wells=4, seed=3), cols, ld, torch.float64)
 
 
+@pytest.mark.parametrize("kind", ["lines", "thin16", "permuted", "permuted13", "thin13"])
+@pytest.mark.parametrize("cols,dtype", [(45, torch.float64), (71, torch.float64),
+                                        (227, torch.float64), (50, torch.float32),
+                                        (98, torch.float32), (258, torch.float32),
+                                        (322, torch.float32)])
+def test_narrow_vectors(kind, cols, dtype):
+    """Rows that start at multiples of 8 bytes only: FP32 in 8-byte vectors, FP64 by elements."""
+    _check(_operator(kind), cols, cols, dtype)
+
+
 @pytest.mark.parametrize("stencil,nev,block", [("star1", 48, 72), ("star1", 100, 136),
                                                ("star2", 72, 100)])
 def test_refined_filter_correction(stencil, nev, block):
