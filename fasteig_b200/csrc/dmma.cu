@@ -324,13 +324,21 @@ namespace {
 // Column tile of the rotation: the one that multiplies least past the output's columns and,
 // for an upper triangular C, below its diagonal; all reach 28 to 30 TFLOP/s, so ties go to
 // the first here. 512,000 rows, k = m: 288 columns 3.30 ms in tiles of 64, 2.87 in tiles of
-// 96; 160 columns 1.14 -> 0.94 ms (32).
-int rotate_tile(int64_t k, int64_t m, bool upper_tri) {
-  constexpr int kTiles[] = {96, 32, 80, 48};
-  int best = 32;
+// 96; 160 columns 1.14 -> 0.94 ms (32). Outputs that are stored one value at a time take a
+// tie's 32 columns, or with many tiles and a short sum 64 (us in tiles of 64 and of 32: 1000
+// rows, 97 columns 22, 15; 40,000 68, 62; 400,000 497, 542; 40,000 x 161 130, 138; 400,000 x
+// 200 x 99 added to the output 971, 868).
+int rotate_tile(int64_t n, int64_t k, int64_t m, bool upper_tri, bool pairs) {
+  constexpr int kPaired[] = {96, 32, 80, 48}, kLong[] = {64, 32, 96, 80, 48},
+                kShort[] = {32, 64, 96, 80, 48};
+  const bool many = (n + kRRows - 1) / kRRows * ((m + 63) / 64) >= 800;
+  const int* kTiles = pairs ? kPaired : many && k <= 176 ? kLong : kShort;
+  const int count = pairs ? 4 : 5;
+  int best = 96;
   int64_t least = -1;
-  for (int t : kTiles) {
-    if (least >= 0 && (m + t - 1) / t > 65535) continue;  // the launch's limit
+  for (int i = 0; i < count; ++i) {
+    const int t = kTiles[i];
+    if ((m + t - 1) / t > 65535 && t != 96) continue;  // the launch's limit
     int64_t cost = 0;
     for (int64_t j = 0; j < m; j += t) cost += t * (upper_tri ? std::min<int64_t>(k, j + t) : k);
     if (least < 0 || cost < least) {
@@ -371,7 +379,7 @@ void rotate_dmma(const double* X, int64_t ldx, const double* C, int64_t ldc, dou
                  cudaStream_t s, bool upper_tri, const int32_t* tile_member, int64_t c_stride) {
   const bool vec2 = aligned16(X) && ldx % 2 == 0 && k % 2 == 0;
   const bool pairs = vec2 && aligned16(Y) && ldy % 2 == 0 && m % 2 == 0;
-  const int cols = rotate_tile(k, m, upper_tri);
+  const int cols = rotate_tile(n, k, m, upper_tri, pairs);
   const int64_t row_tiles = (n + kRRows - 1) / kRRows;
   const int64_t col_tiles = (m + cols - 1) / cols;
   FE_REQUIRE(col_tiles <= 65535, "rotate: too many columns");
@@ -392,7 +400,9 @@ void rotate_dmma(const double* X, int64_t ldx, const double* C, int64_t ldc, dou
   (pairs ? run(rotate_dmma_kernel<2, TC_, true>, TC_)                                      \
          : vec2 ? run(rotate_dmma_kernel<2, TC_, false>, TC_)                              \
                 : run(rotate_dmma_kernel<1, TC_, false>, TC_))
-    if (cols == 32) FE_ROT(32);
+    if (cols == 64)
+      vec2 ? run(rotate_dmma_kernel<2, 64, false>, 64) : run(rotate_dmma_kernel<1, 64, false>, 64);
+    else if (cols == 32) FE_ROT(32);
     else if (cols == 48) FE_ROT(48);
     else if (cols == 80) FE_ROT(80);
     else FE_ROT(96);
