@@ -264,7 +264,7 @@ rotate_kernel(const T* __restrict__ X, int64_t ldx, const double* __restrict__ C
 // rows allow it) and over rows, two to sixteen rows of a thread in flight, so that every row
 // is read in full lines and the SM has 64 KB of loads under way. (One warp per 32
 // columns, a value a lane and a row at a time, took 477 us a call for 512,000 x 96 FP64 with B
-// and R, 2.5 TB/s; this takes 223 us, 5.3 TB/s.)
+// and R, 2.5 TB/s; this takes 205 us, 5.8 TB/s.)
 constexpr int kNormThreads = 1024;
 constexpr int kNormMaxVecs = 512;  // vectors of a row that one CTA takes at most
 constexpr int kNormMaxChunks = 148;
